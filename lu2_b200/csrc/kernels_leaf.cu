@@ -311,6 +311,10 @@ static cudaError_t launch_leaf_t(T *a, long ld, int n, int c0, int w, int mode, 
                                  const LeafBuffers &buf, int *status, int max_ctas, cudaStream_t st)
 {
     if (w <= 0) return cudaSuccess;
+    bool used = false;
+    const cudaError_t ce =
+        launch_leaf_cluster(a, ld, n, c0, w, mode, goff, ipiv, dinv, buf, status, max_ctas, st, &used);
+    if (ce != cudaSuccess || used) return ce;
     if (w > LEAF_W) return cudaErrorInvalidValue;
     const int rows = n - c0;
     int G = (rows + LEAF_MIN_ROWS - 1) / LEAF_MIN_ROWS;

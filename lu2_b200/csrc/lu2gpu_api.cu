@@ -98,7 +98,6 @@ struct lu2gpu_ctx {
     LeafBuffers leaf{};
     unsigned long long leaf_seq = 0;  // leaf publication stamps issued so far
     int leaf_ctas = 0;
-    int leaf_w = 16;
     // staging for the host-pointer entry points
     double *d_stage[4] = {nullptr, nullptr, nullptr, nullptr};
     size_t stage_cap[4] = {0, 0, 0, 0};
@@ -498,7 +497,7 @@ static int right_part_split(lu2gpu_ctx *c, const View &v, int k0, int k1, int cs
 // split keeps every left width a multiple of 16 (the GEMM's K step).
 static int panel(lu2gpu_ctx *c, const View &v, int c0, int m, int mode)
 {
-    if (m <= c->leaf_w) {
+    if (m <= leaf_width(v.n - c0, sizeof(double), c->leaf_ctas)) {
         PhaseTimer t(c, PH_LEAF);
         K_TRY(launch_leaf(v.a, v.ld, v.n, c0, m, mode, v.goff, c->d_ipiv + v.goff, c->d_dinv + v.goff, c->leaf,
                           c->d_status, c->leaf_ctas, c->stream));
@@ -2055,7 +2054,7 @@ static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, in
 
 static int panel32(lu2gpu_ctx *c, const View32 &v, int c0, int m, int mode)
 {
-    if (m <= c->leaf_w) {
+    if (m <= leaf_width(v.n - c0, sizeof(float), c->leaf_ctas)) {
         PhaseTimer t(c, PH_LEAF);
         K_TRY(launch_leaf(v.a, v.ld, v.n, c0, m, mode, v.goff, c->d_ipiv + v.goff, c->mx->dinv + v.goff, c->leaf,
                           c->d_status, c->leaf_ctas, c->stream));

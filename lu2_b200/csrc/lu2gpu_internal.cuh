@@ -113,7 +113,7 @@ struct LeafBuffers {
     int withhold = -1;
 };
 
-// Factor the leaf panel: rows c0..n-1, columns c0..c0+w-1 (w <= 16) of the
+// Factor the leaf panel: rows c0..n-1, columns c0..c0+w-1 (w <= leaf_width) of the
 // view `a` whose element (0,0) is global (goff, goff).  ipiv/dinv are indexed
 // by view column; ipiv receives global row numbers (view row + goff).
 cudaError_t launch_leaf(double *a, long ld, int n, int c0, int w, int mode, int goff, int *ipiv, double *dinv,
@@ -121,6 +121,14 @@ cudaError_t launch_leaf(double *a, long ld, int n, int c0, int w, int mode, int 
 cudaError_t launch_leaf(float *a, long ld, int n, int c0, int w, int mode, int goff, int *ipiv, float *dinv,
                         const LeafBuffers &buf, int *status, int max_ctas, cudaStream_t st);
 int leaf_max_ctas(int device);
+// widest leaf for a panel of `rows` rows (elements of tsize bytes) with at most max_ctas CTAs
+int leaf_width(int rows, size_t tsize, int max_ctas);
+// the leaf on one thread-block cluster (kernels_cleaf.cu); *used = false, and
+// nothing launched, where it does not take the panel
+cudaError_t launch_leaf_cluster(double *a, long ld, int n, int c0, int w, int mode, int goff, int *ipiv, double *dinv,
+                                const LeafBuffers &buf, int *status, int max_ctas, cudaStream_t st, bool *used);
+cudaError_t launch_leaf_cluster(float *a, long ld, int n, int c0, int w, int mode, int goff, int *ipiv, float *dinv,
+                                const LeafBuffers &buf, int *status, int max_ctas, cudaStream_t st, bool *used);
 // fewest leaf CTAs whose slabs of `rows` rows (elements of tsize bytes) fit shared memory
 int leaf_min_ctas(int rows, size_t tsize);
 
