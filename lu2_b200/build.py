@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "liblu2gpu.so")
-SOURCES = ["kernels_leaf.cu", "kernels_cleaf.cu", "kernels_panel.cu", "kernels_dgemm.cu", "kernels_solve.cu", "kernels_bf16.cu", "kernels_mixed.cu",
+SOURCES = ["kernels_leaf.cu", "kernels_cleaf.cu", "kernels_panel.cu", "kernels_dgemm.cu", "kernels_solve.cu", "kernels_trisolve.cu", "kernels_bf16.cu", "kernels_mixed.cu",
            "kernels_batch.cu", "kernels_batch_ir.cu", "kernels_fp8.cu", "kernels_lowp.cu", "kernels_gmres.cu",
            "lu2gpu_api.cu"]
 HEADERS = ["lu2gpu_internal.cuh"]

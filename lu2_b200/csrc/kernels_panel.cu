@@ -321,6 +321,55 @@ cudaError_t launch_laswp_scale(float *a, long ld, int nrows, int k0, int k1, con
 }
 
 // ---------------------------------------------------------------------------
+// The row maps of the forward solve with stored factors (kernels_trisolve.cu).
+// One CTA per panel P writes inv[P][q] = the position, before the panel's
+// exchanges, of the row they leave at position q (the composed permutation);
+// then each final position f walks back through the panels up to its own.
+__global__ void __launch_bounds__(SWAP_THREADS) solve_inv_kernel(const int *__restrict__ ipiv, int n, int nb, int *inv,
+                                                                 int *status)
+{
+    extern __shared__ __align__(16) int plan_smem[];
+    __shared__ int s_nslot, s_bad;
+    const int k0 = blockIdx.x * nb, k1 = min(n, k0 + nb), npiv = k1 - k0;
+    int *P = plan_smem, *A = P + npiv, *src = A + npiv, *dst = src + 2 * npiv;
+    // (one decision for the CTA; swap_plan without status neither looks nor records)
+    if (__syncthreads_or(threadIdx.x == 0 && *(volatile int *)&status[1] != 0)) return;
+    if (!swap_plan(ipiv, 0, k0, k1, n, P, A, src, dst, &s_nslot, &s_bad, nullptr)) {
+        if (threadIdx.x == 0) record_error(status, ERR_BAD_ARG, 3);
+        return;
+    }
+    int *row = inv + (size_t)blockIdx.x * n;
+    for (int q = k0 + threadIdx.x; q < n; q += blockDim.x) row[q] = q;
+    __syncthreads();
+    for (int i = threadIdx.x; i < s_nslot; i += blockDim.x) row[dst[i]] = src[i];
+}
+
+__global__ void __launch_bounds__(SWAP_THREADS) solve_rows_kernel(const int *__restrict__ inv, int n, int nb, int *rows,
+                                                                  const int *status)
+{
+    if (*(volatile const int *)&status[1] != 0) return;  // maps are missing
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= n) return;
+    int pos = f;
+    for (int P = f / nb; P >= 0; P--) {
+        pos = inv[(size_t)P * n + pos];
+        rows[(size_t)P * n + f] = pos;
+    }
+}
+
+cudaError_t launch_solve_plan(const int *ipiv, int n, int nb, int *inv, int *rows, int *status, cudaStream_t st)
+{
+    if (n <= 0 || nb <= 0 || nb > SWAP_MAX_PIV) return cudaErrorInvalidValue;
+    const int npan = (n + nb - 1) / nb;
+    count_launch(2);
+    solve_inv_kernel<<<npan, SWAP_THREADS, (size_t)6 * nb * sizeof(int), st>>>(ipiv, n, nb, inv, status);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    solve_rows_kernel<<<(n + SWAP_THREADS - 1) / SWAP_THREADS, SWAP_THREADS, 0, st>>>(inv, n, nb, rows, status);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
 // Unit-lower triangular solve of a 32-column strip of the block row, staged
 // in shared memory.  T is consumed in 16-column blocks: each block of T
 // (rows lb..K-1) is first copied to shared memory with coalesced 128-byte row

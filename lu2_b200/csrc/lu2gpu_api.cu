@@ -116,27 +116,31 @@ struct lu2gpu_ctx {
     long launches[PH_COUNT] = {};
     // workspaces of the precision form (lu2gpu_mixed_solve), allocated on first use
     struct MixedWork *mx = nullptr;
-    // stamped x slots of the persistent back substitution (one per 64-row block)
+    // stamped x slots of the persistent triangular solves
     unsigned long long *d_bsx = nullptr;
-    int bsx_cap = 0;
+    int bsx_cap = 0;  // rows
     unsigned bs_epoch = 0;
     BsBuffers bs{};
+    // the forward solve with stored factors: row maps (two [panels][n] arrays), transformed right-hand sides
+    int *d_plan = nullptr;
+    size_t plan_cap = 0;
+    double *d_fwd = nullptr;
+    size_t fwd_cap = 0;
 };
 
 static void free_mixed(lu2gpu_ctx *c);
 
-// the back substitution's x slots for an order-n system (null when they
-// cannot be had: the blocked launches then do it)
+// the x slots of the persistent triangular solves of an order-n system (null
+// when they cannot be had: the blocked launches then do it)
 static const BsBuffers *bs_buffers(lu2gpu_ctx *c, int n)
 {
     if (c->fixed_scratch) return nullptr;
-    const int need = (n + 63) / 64;
-    if (need > c->bsx_cap) {
+    if (n > c->bsx_cap) {
         cudaFree(c->d_bsx);
         c->d_bsx = nullptr;
         c->bsx_cap = 0;
-        const int cap = need + 256;
-        const size_t bytes = (size_t)cap * BS_SLOT_WORDS * sizeof(unsigned long long);
+        const int cap = n + n / 8 + 1024;
+        const size_t bytes = (size_t)cap * BS_ROW_WORDS * sizeof(unsigned long long);
         if (cudaMalloc(&c->d_bsx, bytes) != cudaSuccess || cudaMemsetAsync(c->d_bsx, 0, bytes, c->stream) != cudaSuccess) {
             cudaGetLastError();
             cudaFree(c->d_bsx);
@@ -146,7 +150,7 @@ static const BsBuffers *bs_buffers(lu2gpu_ctx *c, int n)
         c->bsx_cap = cap;
     }
     c->bs.xslots = c->d_bsx;
-    c->bs.cap = c->bsx_cap;
+    c->bs.cap_rows = c->bsx_cap;
     c->bs.epoch = &c->bs_epoch;
     c->bs.status = c->d_status;
     return &c->bs;
@@ -180,6 +184,21 @@ static int grow(void **p, size_t *cap, size_t bytes)
     }
     *cap = bytes;
     return 0;
+}
+
+// The persistent forward solve's map for the pivots ipiv (device) and panel
+// width nb, enqueued; null where its buffers cannot be had (the solve then
+// goes panel by panel).
+static const int *solve_rows(lu2gpu_ctx *c, int n, int nb, const int *ipiv)
+{
+    const size_t each = ((size_t)n + nb - 1) / nb * n;
+    if (!bs_buffers(c, n) || grow((void **)&c->d_plan, &c->plan_cap, 2 * each * sizeof(int)) ||
+        grow((void **)&c->d_fwd, &c->fwd_cap, (size_t)n * BS_MAXR * sizeof(double)) ||
+        launch_solve_plan(ipiv, n, nb, c->d_plan + each, c->d_plan, c->d_status, c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return c->d_plan;
 }
 
 static int stage(lu2gpu_ctx *c, int slot, size_t doubles, double **out)
@@ -265,6 +284,8 @@ extern "C" int lu2gpu_destroy(lu2gpu_ctx *c)
     cudaFree(c->d_ipiv);
     cudaFree(c->d_dinv);
     cudaFree(c->d_bsx);
+    cudaFree(c->d_plan);
+    cudaFree(c->d_fwd);
     for (int i = 0; i < 4; i++) cudaFree(c->d_stage[i]);
     if (c->copy_stream) {
         cudaStreamSynchronize(c->copy_stream);
@@ -795,6 +816,10 @@ extern "C" int lu2gpu_lusolve(lu2gpu_ctx *c, int n, int nrhs, double *a, long ld
 // unit-lower solve and the update of the rows below -- what the factorization
 // does to its augmented columns (lu2.c:524-581) -- then the back substitution
 // (lu2.c:110-116).  b (n x nrhs, row stride ldb) is overwritten by x.
+// Up to SOLVE_FEW_RHS right-hand sides go through the two persistent solves,
+// eight at a time; more through one panel loop whose products take them all.
+constexpr int SOLVE_FEW_RHS = 32;
+
 extern "C" int lu2gpu_solve(lu2gpu_ctx *c, int n, const double *a, long lda, int nb, const int *ipiv, double *b,
                             long ldb, int nrhs)
 {
@@ -809,6 +834,24 @@ extern "C" int lu2gpu_solve(lu2gpu_ctx *c, int n, const double *a, long lda, int
     if ((rc = ensure_work(c, n, nrhs, nb))) return rc;
     if ((rc = begin_status(c))) return rc;
     K_TRY(launch_diag_inv(a, lda, n, c->d_dinv, c->stream));
+    const int *rows = nrhs <= SOLVE_FEW_RHS ? solve_rows(c, n, nb, ipiv) : nullptr;
+    if (rows) {
+        bool used = false;
+        for (int q = 0; q < nrhs; q += BS_MAXR) {
+            const int nr = std::min(BS_MAXR, nrhs - q);
+            K_TRY(launch_lower_solve(a, lda, n, nb, rows, c->d_dinv, b + q, ldb, nr, c->d_fwd, nr, c->bs, c->stream,
+                                     &used));
+            if (!used) break;  // the first chunk decides: all have the same blocks
+            bool up = false;
+            PhaseTimer t(c, PH_BACKSOLVE);
+            K_TRY(launch_upper_solve(a, lda, n, nr, c->d_fwd, nr, b + q, ldb, c->bs, c->stream, &up));
+            if (!up) {
+                set_error("lu2gpu_solve: the back substitution does not fit the device (n=%d)", n);
+                return LU2GPU_ERR_ARG;
+            }
+        }
+        if (used) return end_status(c, "lu2gpu_solve");
+    }
     for (int i = 0; i < n; i += nb) {
         const int w = (n - i) < nb ? (n - i) : nb;
         K_TRY(launch_laswp_scale(b, ldb, n, i, i + w, ipiv, 0, c->d_dinv, 0, nrhs, true, c->d_status, c->stream));
@@ -2074,9 +2117,20 @@ static int panel32(lu2gpu_ctx *c, const View32 &v, int c0, int m, int mode)
 
 // FP32 forward solve with the stored factors (what the factorization applies
 // to an augmented column, panel by panel), then the back substitution.
-static int solve32_enqueue(lu2gpu_ctx *c, int n, const float *a, long ld, int nb, float *v)
+static int solve32_enqueue(lu2gpu_ctx *c, int n, const float *a, long ld, int nb, const int *rows, float *v)
 {
     MixedWork *m = c->mx;
+    if (rows) {  // two persistent launches (c->d_fwd and the slots come with the map)
+        bool used = false;
+        float *y = reinterpret_cast<float *>(c->d_fwd);
+        K_TRY(launch_lower_solve(a, ld, n, nb, rows, m->dinv, v, 1, 1, y, 1, c->bs, c->stream, &used));
+        if (used) {
+            K_TRY(launch_upper_solve(a, ld, n, 1, y, 1, v, 1, c->bs, c->stream, &used));
+            if (used) return 0;
+            set_error("the back substitution does not fit the device (n=%d)", n);
+            return LU2GPU_ERR_ARG;
+        }
+    }
     for (int i = 0; i < n; i += nb) {
         const int w = (n - i) < nb ? (n - i) : nb;
         K_TRY(launch_laswp_scale(v, 1, n, i, i + w, c->d_ipiv, 0, m->dinv, 0, 1, true, c->d_status, c->stream));
@@ -2747,6 +2801,7 @@ extern "C" int lu2gpu_mixed_solve(lu2gpu_ctx *c, int n, const double *a, long ld
     if ((rc = factor32_or_fail(c, n, m->a32, ld32, nb, pivot_mode))) return rc;
     CU_TRY(cudaEventRecord(ev[1], c->stream));
 
+    const int *rows = solve_rows(c, n, nb, c->d_ipiv);
     // refinement: x_0 = 0, r_0 = b; d = LU^{-1} r (FP32), x += d, r = b - A x (FP64)
     CU_TRY(cudaMemsetAsync(x, 0, (size_t)n * sizeof(double), c->stream));
     CU_TRY(cudaMemcpyAsync(r, b, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
@@ -2755,7 +2810,7 @@ extern "C" int lu2gpu_mixed_solve(lu2gpu_ctx *c, int n, const double *a, long ld
     int it = 0;
     for (it = 1; it <= max_iter; it++) {
         K_TRY(launch_f64_to_f32(r, 1, v32, 1, n, 1, c->stream));
-        if ((rc = solve32_enqueue(c, n, m->a32, ld32, nb, v32))) return rc;
+        if ((rc = solve32_enqueue(c, n, m->a32, ld32, nb, rows, v32))) return rc;
         K_TRY(launch_add_f32_to_f64(v32, x, n, c->stream));
         K_TRY(launch_residual(a, lda, n, b, x, r, it == 1 ? rowabs : nullptr, c->stream));
         CU_TRY(cudaMemsetAsync(m->norms(), 0, (it == 1 ? 4 : 2) * sizeof(unsigned long long), c->stream));
@@ -2799,12 +2854,12 @@ extern "C" int lu2gpu_mixed_solve(lu2gpu_ctx *c, int n, const double *a, long ld
 // GMRES-IR
 
 // z = U^{-1} L^{-1} P w with the FP32 factors (FP64 vectors in and out)
-static int precond_apply(lu2gpu_ctx *c, int n, long ld32, int nb, const double *w, double *z)
+static int precond_apply(lu2gpu_ctx *c, int n, long ld32, int nb, const int *rows, const double *w, double *z)
 {
     MixedWork *m = c->mx;
     float *v32 = reinterpret_cast<float *>(m->vec + 3 * (size_t)n);
     K_TRY(launch_f64_to_f32(w, 1, v32, 1, n, 1, c->stream));
-    int rc = solve32_enqueue(c, n, m->a32, ld32, nb, v32);
+    int rc = solve32_enqueue(c, n, m->a32, ld32, nb, rows, v32);
     if (rc) return rc;
     K_TRY(launch_f32_to_f64(v32, 1, z, 1, n, 1, c->stream));
     return 0;
@@ -2892,6 +2947,7 @@ extern "C" int lu2gpu_gmres_solve(lu2gpu_ctx *c, int n, const double *a, long ld
     if ((rc = factor32_or_fail(c, n, m->a32, ld32, nb, LU2GPU_PIVOT_PARTIAL))) return rc;
     CU_TRY(cudaEventRecord(ev[1], c->stream));
 
+    const int *rows = solve_rows(c, n, nb, c->d_ipiv);
     const double one = 1.0;
     CU_TRY(cudaMemcpyAsync(dots + 128, &one, sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CU_TRY(cudaMemsetAsync(x, 0, (size_t)n * sizeof(double), c->stream));
@@ -2934,7 +2990,7 @@ extern "C" int lu2gpu_gmres_solve(lu2gpu_ctx *c, int n, const double *a, long ld
         outer++;
         // correction equation A d = r, left-preconditioned: M^{-1} A d = M^{-1} r
         CU_TRY(cudaMemsetAsync(d, 0, (size_t)n * sizeof(double), c->stream));
-        if ((rc = precond_apply(c, n, ld32, nb, r, z))) return rc;
+        if ((rc = precond_apply(c, n, ld32, nb, rows, r, z))) return rc;
         double beta0 = 0;
         if ((rc = norm_of(z, &beta0))) return rc;
         if (!std::isfinite(beta0)) {  // the FP32 solve with the low-precision factors overflowed
@@ -2952,7 +3008,7 @@ extern "C" int lu2gpu_gmres_solve(lu2gpu_ctx *c, int n, const double *a, long ld
             while (k < restart && total < max_iter) {
                 double *vk = V + (size_t)k * ldv;
                 K_TRY(launch_residual(a, lda, n, nullptr, vk, w, nullptr, c->stream));  // w = A v_k
-                if ((rc = precond_apply(c, n, ld32, nb, w, z))) return rc;
+                if ((rc = precond_apply(c, n, ld32, nb, rows, w, z))) return rc;
                 // classical Gram-Schmidt, twice
                 K_TRY(launch_multi_dot(V, ldv, k + 1, z, n, partial, dots, c->stream));
                 K_TRY(launch_multi_axpy(V, ldv, k + 1, dots, -1.0, z, n, c->stream));
@@ -2998,7 +3054,7 @@ extern "C" int lu2gpu_gmres_solve(lu2gpu_ctx *c, int n, const double *a, long ld
             if (!conv && total < max_iter) {
                 // restart from the true correction residual r - A d
                 K_TRY(launch_residual(a, lda, n, r, d, t, nullptr, c->stream));
-                if ((rc = precond_apply(c, n, ld32, nb, t, z))) return rc;
+                if ((rc = precond_apply(c, n, ld32, nb, rows, t, z))) return rc;
                 if ((rc = norm_of(z, &beta))) return rc;
                 if (!(beta > inner_tol * beta0)) conv = true;
             }

@@ -174,23 +174,42 @@ cudaError_t launch_transpose(const double *in, long ldi, double *out, long ldo, 
 
 // x = U'^{-1} y for the unit upper triangle of a[0..n)[0..n) (lu2's backward_sub,
 // lu2.c:110-116); y (n x nrhs, row stride ldx) is overwritten by x.  For lu2's
-// own layout x = a + n, ldx = ld.  With bs (a stamped x slot for each of the
-// n / 64 blocks, zeroed once; a host epoch counter; the status words) and
-// n >= BSP_PERSISTENT_MIN_N one persistent cooperative launch per 8
-// right-hand sides does it; otherwise blocked launches (one per 128-row block
-// and one per update).
-constexpr int BS_SLOT_WORDS = 64 * 8 * 2;  // 64 rows x 8 right-hand sides, two stamped words each
+// own layout x = a + n, ldx = ld.  With bs (stamped x slots, zeroed once; a
+// host epoch counter; the status words) one persistent cooperative launch per
+// BS_MAXR right-hand sides does it (kernels_trisolve.cu); otherwise blocked
+// launches (one per 128-row block and one per update).
+constexpr int BS_MAXR = 8;                    // right-hand sides handled per pass
+constexpr int BS_ROW_WORDS = BS_MAXR * 2;     // slot words of a row: two stamped words per element
 struct BsBuffers {
-    unsigned long long *xslots = nullptr;  // [cap][BS_SLOT_WORDS], zeroed at allocation
-    int cap = 0;
+    unsigned long long *xslots = nullptr;  // [cap_rows][BS_ROW_WORDS], zeroed at allocation
+    int cap_rows = 0;
     unsigned *epoch = nullptr;  // host-side counter, advanced per launch
     int *status = nullptr;
 };
-constexpr int BSP_PERSISTENT_MIN_N = 4096;
 cudaError_t launch_backsolve(const double *a, long ld, int n, int nrhs, double *x, long ldx, const BsBuffers *bs,
                              cudaStream_t st);
 cudaError_t launch_backsolve(const float *a, long ld, int n, int nrhs, float *x, long ldx, const BsBuffers *bs,
                              cudaStream_t st);
+// The persistent solves (kernels_trisolve.cu); *used = false, and nothing
+// launched, where a solve does not fit.  Upper as above with y apart from x
+// (x may be y).  Lower: y = the forward-transformed b (nrhs <= BS_MAXR) for
+// factors of panel width nb; rows is launch_solve_plan's map, dinv 1/pivot;
+// y may not overlap b.
+cudaError_t launch_upper_solve(const double *a, long ld, int n, int nrhs, const double *y, long ldy, double *x, long ldx,
+                               const BsBuffers &bs, cudaStream_t st, bool *used);
+cudaError_t launch_upper_solve(const float *a, long ld, int n, int nrhs, const float *y, long ldy, float *x, long ldx,
+                               const BsBuffers &bs, cudaStream_t st, bool *used);
+cudaError_t launch_lower_solve(const double *a, long ld, int n, int nb, const int *rows, const double *dinv,
+                               const double *b, long ldb, int nrhs, double *y, long ldy, const BsBuffers &bs,
+                               cudaStream_t st, bool *used);
+cudaError_t launch_lower_solve(const float *a, long ld, int n, int nb, const int *rows, const float *dinv,
+                               const float *b, long ldb, int nrhs, float *y, long ldy, const BsBuffers &bs,
+                               cudaStream_t st, bool *used);
+// rows[P][f] (P < ceil(n / nb)): the position, before panel P's exchanges, of
+// the row that ends at position f >= P nb of the whole sequence ipiv (0-based,
+// row k exchanged with ipiv[k] >= k).  inv: scratch of the same size.  A pivot
+// outside [k, n) sets ERR_BAD_ARG in status[1].
+cudaError_t launch_solve_plan(const int *ipiv, int n, int nb, int *inv, int *rows, int *status, cudaStream_t st);
 
 // out[k] = 1 / a[k][k] (1 for an exactly zero pivot)
 cudaError_t launch_diag_inv(const double *a, long ld, int n, double *out, cudaStream_t st);
