@@ -23,19 +23,26 @@
 // (bounded wait), which gives it x in the same round trip.
 //
 // What bounds it: the chain of blocks, one solve, one publication and one
-// tile product each -- not the factor's bytes.  Hence 128 rows a block (the
-// publication, about 1.5 us through L2, is paid half as often as with 64), and
-// the diagonal block solved four columns at a time: their four values are
-// shuffled to all lanes together and finished there redundantly, so a column
-// costs a quarter of a shuffle's latency.
+// tile product each -- not the factor's bytes.  Hence
+//  * 128 rows a block: the publication, about 1 us through L2, is paid half as
+//    often as with 64;
+//  * a block's solve runs in four warps per right-hand side, 32 rows each: a
+//    warp finishes its triangle four columns at a time (their values shuffled
+//    to all lanes together and finished there redundantly, so that a column
+//    costs a quarter of a shuffle's latency), then the later warps subtract its
+//    32 columns.  One warp walking all 128 rows took 11800 cycles a block;
+//  * FP64 tile products run on the tensor pipe (mma.sync m16n8k8, always eight
+//    right-hand sides wide, so that a column's result does not depend on how
+//    many there are): read from shared memory by every thread, x cost 8600
+//    cycles a block with 4 right-hand sides; the tensor pipe takes 2050 with
+//    any number, the CUDA cores 1250 with one.
 //
 // The FP64 lower solve repeats the factorization's own operations on a riding
 // column in the same order, so that a re-solve gives what the factorization
 // gave (with the shipped reference's pivots anything else differs visibly):
 // inside a panel the 16-row blocks of trsm_dmma_kernel (16 products summed
-// from zero, then subtracted), across panels one chain of multiply-adds per
-// element in the trailing update's order.  The chain runs through the four
-// threads of a row, 32 columns each, one right-hand side behind the other.
+// from zero, then subtracted), across panels the trailing update's own MMA
+// with its permuted k, accumulating on the right-hand side column after column.
 //
 // The lower solve's rows.  Earlier panels' L columns are not swapped by later
 // panels (lu2.c:543-553): the row that ends at position f sat at position
@@ -48,10 +55,10 @@
 namespace lu2gpu {
 
 constexpr int TS_B = 128;         // rows per block
-constexpr int TS_THREADS = 512;   // four threads per row of a tile
+constexpr int TS_THREADS = 512;
 constexpr int TS_TLD = TS_B + 1;  // pitch of the diagonal block in shared memory
 constexpr int TS_E = TS_B / 4;    // elements of a tile per thread
-constexpr int TS_XBUF = TS_B + 8;  // a source's x per right-hand side, padded
+constexpr int TS_XQ = TS_B + 8;   // pitch of a source's x per right-hand side: B fragments on distinct banks
 
 template <typename T>
 struct TriParams {
@@ -84,21 +91,47 @@ __device__ __forceinline__ void ts_ld2(const float *p, float &a, float &b)
     b = w.y;
 }
 
+__device__ __forceinline__ unsigned ts_smem32(const void *p)
+{
+    return static_cast<unsigned>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void ts_lds(unsigned p, double &v) { asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(p)); }
+__device__ __forceinline__ void ts_lds(unsigned p, float &v) { asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(p)); }
+__device__ __forceinline__ void ts_lds2(unsigned p, double &a, double &b)
+{
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "r"(p));
+}
+__device__ __forceinline__ void ts_lds2(unsigned p, float &a, float &b)
+{
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(p));
+}
+
+__device__ __forceinline__ void ts_mma(double (&c)[4], double a0, double a1, double a2, double a3, double b0, double b1)
+{
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};\n"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
+}
+
+// NR = 1 (FP32): one right-hand side on the CUDA cores; NR = 8 (FP64): up to 8,
+// padded with zeros, on the tensor pipe.  EXACT: the FP64 lower solve.
 template <typename T, bool LOWER, int NR>
 __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParams<T> P)
 {
-    constexpr bool EXACT = LOWER && sizeof(T) == 8;  // the factorization's order of operations
-    constexpr int XQ = EXACT ? TS_B + 8 : 1, XB = TS_XBUF * NR;
-    // element (row c, right-hand side q) of a source's x: for the chain by
-    // right-hand side, padded so that the four threads of a row hit distinct banks
-    auto xi = [](int c, int q) { return EXACT ? q * XQ + c + 2 * (c >> 5) : c * NR + q; };
+    constexpr bool MMA = NR == 8, EXACT = LOWER && sizeof(T) == 8;
+    static_assert(!EXACT || MMA, "the factorization's order of operations is the MMA's");
+    static_assert(!MMA || sizeof(T) == 8, "FP64 MMA");
     extern __shared__ __align__(16) unsigned char ts_smem[];
     const int G = gridDim.x, cta = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nblk = P.nblk;
     const int n_own = cta < nblk ? (nblk - cta + G - 1) / G : 0;
-    T *Td = reinterpret_cast<T *>(ts_smem);   // [TS_B][TS_TLD], the owned diagonal block solved next
-    T *xs = Td + TS_B * TS_TLD;  // [2][TS_XBUF NR]
-    T *acc = xs + 2 * XB;                     // [n_own][TS_B][NR]
+    constexpr int XB = TS_XQ * NR;
+    T *Td = reinterpret_cast<T *>(ts_smem);      // [TS_B][TS_TLD], the owned diagonal block solved next
+    T *xs = Td + TS_B * TS_TLD;                  // [2][NR][TS_XQ]
+    T *part_sum = xs + 2 * XB;                   // [TS_B][NR] (tensor pipe, not EXACT)
+    T *acc = part_sum + (MMA && !EXACT ? TS_B * NR : 0);  // [n_own][TS_B][NR]
     T *sdinv = acc + (size_t)n_own * TS_B * NR;  // [n_own][TS_B] (lower)
     // an earlier wait or check of this call failed: nothing to do
     if (__syncthreads_or(tid == 0 && *(volatile int *)&P.status[1] != 0)) return;
@@ -131,6 +164,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParam
             for (int r = tid; r < TS_B; r += TS_THREADS)
                 sdinv[k * TS_B + r] = r < rows ? P.dinv[r0 + r] : T(1);
     }
+    for (int e = tid; e < 2 * XB; e += TS_THREADS) xs[e] = T(0);  // right-hand sides past nr stay zero
 
     // owned block k's diagonal block into Td (issued right after the previous
     // solve, off the critical path), zero outside its strict triangle
@@ -156,193 +190,269 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParam
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    // solve owned block k (all updates applied) into xs[buf] and x; one warp
-    // per right-hand side, lane l holding rows l, l + 32, l + 64, l + 96
+    // solve owned block k (all updates applied) into xs[buf] and x: four warps
+    // per right-hand side q (then q + 4), warp m of them with rows 32 m ..
+    // 32 m + 31, one per lane.  (m is rotated with q: the warps whose turn it
+    // is at the same time sit on different schedulers.)
     auto solve = [&](int k, int buf) {
         const int p = cta + k * G, r0 = r0_of(p), rows = rows_of(p);
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        if (warp < NR && warp < P.nr) {
-            T y[4];
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                const int r = 32 * m + lane;
-                y[m] = acc[((size_t)k * TS_B + r) * NR + warp];
-                if (LOWER && p % P.bpp == 0) y[m] *= sdinv[k * TS_B + r];  // a panel's first block: nothing scaled it yet
-            }
-#pragma unroll
-            for (int mm = 0; mm < 4; mm++) {
-                const int mo = LOWER ? mm : 3 - mm;  // the rows being finished
-                T s[4];  // EXACT: a 16-column block's products, subtracted together
+        const int m = (warp + (warp >> 2)) & 3, r = 32 * m + lane;
+        const unsigned td = ts_smem32(Td), tr = td + r * TS_TLD * (unsigned)sizeof(T);
+        unsigned long long *slot = P.xslots + (size_t)r0 * (2 * BS_MAXR);
 #pragma unroll 1
-                for (int ll = 0; ll < 32; ll += 4) {
-                    const int l0 = LOWER ? ll : 28 - ll, c0 = 32 * mo + l0;
-                    if (c0 >= rows) continue;
-                    // the four columns c0..c0+3 in solve order: e-th is column ce(e)
-                    T xv[4];
+        for (int q = warp >> 2; q < NR && q < P.nr; q += 4) {
+            T *X = xs + buf * XB + q * TS_XQ;
+            const unsigned xq = ts_smem32(X);
+            T y = acc[((size_t)k * TS_B + r) * NR + q];
+            if (LOWER && p % P.bpp == 0) y *= sdinv[k * TS_B + r];  // a panel's first block: nothing scaled it yet
+#pragma unroll 1
+            for (int jj = 0; jj < 4; jj++) {
+                const int j = LOWER ? jj : 3 - jj;  // the warp whose turn it is
+                if (32 * j >= rows) continue;
+                if (m == j) {
+                    T s = T(0);  // EXACT: the first 16 columns' products for the later 16 rows
+                    // group ll's columns in solve order, the lane's row and the 4 x 4 triangle,
+                    // read one group ahead
+                    T tc[4], tt[6];
+                    auto fetch = [&](int ll) {
+                        const int c0 = 32 * j + (LOWER ? ll : 28 - ll);
 #pragma unroll
-                    for (int e = 0; e < 4; e++) xv[e] = __shfl_sync(0xffffffffu, y[mo], l0 + (LOWER ? e : 3 - e));
+                        for (int e = 0; e < 4; e++) ts_lds(tr + (c0 + (LOWER ? e : 3 - e)) * (unsigned)sizeof(T), tc[e]);
 #pragma unroll
-                    for (int e = 1; e < 4; e++)
+                        for (int e = 1; e < 4; e++)
 #pragma unroll
-                        for (int f = 0; f < e; f++) {
-                            const int re = c0 + (LOWER ? e : 3 - e), cf = c0 + (LOWER ? f : 3 - f);
-                            xv[e] -= Td[re * TS_TLD + cf] * xv[f];
-                        }
-                    // the other rows; of block mo the lanes beyond the four
+                            for (int f = 0; f < e; f++) {
+                                const int re = c0 + (LOWER ? e : 3 - e), cf = c0 + (LOWER ? f : 3 - f);
+                                ts_lds(td + (re * TS_TLD + cf) * (unsigned)sizeof(T), tt[e * (e - 1) / 2 + f]);
+                            }
+                    };
+                    fetch(0);
 #pragma unroll
-                    for (int m = 0; m < 4; m++) {
-                        if (LOWER ? m < mo : m > mo) continue;
-                        // rows after the 16-column block (EXACT): from zero at the block's first columns
-                        const bool far = EXACT && (m != mo || (ll < 16 && lane >= 16));
-                        T v = y[m];
-                        if (far) v = (ll & 15) == 0 ? T(0) : s[m];
-                        const T *tr = Td + (32 * m + lane) * TS_TLD + c0;
+                    for (int ll = 0; ll < 32; ll += 4) {
+                        const int l0 = LOWER ? ll : 28 - ll;
+                        T xv[4], cc[4], ct[6];
 #pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const T t = tr[LOWER ? e : 3 - e];
-                            v = fma(far ? t : -t, xv[e], v);
-                        }
-                        if (far) {
-                            s[m] = v;
-                            if ((ll & 15) == 12 || c0 + 4 >= rows) y[m] -= v;
-                        } else if (m != mo) {
-                            y[m] = v;
-                        } else {
-                            if (LOWER ? lane > l0 + 3 : lane < l0) y[m] = v;
+                        for (int e = 0; e < 4; e++) xv[e] = __shfl_sync(0xffffffffu, y, l0 + (LOWER ? e : 3 - e));
 #pragma unroll
-                            for (int e = 0; e < 4; e++)
-                                if (lane == l0 + (LOWER ? e : 3 - e)) y[m] = xv[e];
-                        }
+                        for (int e = 0; e < 4; e++) cc[e] = tc[e];
+#pragma unroll
+                        for (int e = 0; e < 6; e++) ct[e] = tt[e];
+                        if (ll + 4 < 32) fetch(ll + 4);
+#pragma unroll
+                        for (int e = 1; e < 4; e++)
+#pragma unroll
+                            for (int f = 0; f < e; f++) xv[e] = fma(-ct[e * (e - 1) / 2 + f], xv[f], xv[e]);
+                        const bool far = EXACT && ll < 16 && lane >= 16;
+                        T v = far ? s : y;
+#pragma unroll
+                        for (int e = 0; e < 4; e++) v = fma(far ? cc[e] : -cc[e], xv[e], v);
+                        s = far ? v : s;
+                        const T yf = y - s;
+                        y = far ? (ll == 12 ? yf : y) : ((LOWER ? lane > l0 + 3 : lane < l0) ? v : y);
+#pragma unroll
+                        for (int e = 0; e < 4; e++) y = lane == l0 + (LOWER ? e : 3 - e) ? xv[e] : y;
                     }
+                    X[r] = r < rows ? y : T(0);
+                }
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + (warp >> 2)) : "memory");
+                if (LOWER ? m > j : m < j) {
+                    // two chains of 16 products
+                    const unsigned tj = tr + 32 * j * (unsigned)sizeof(T), xj = xq + 32 * j * (unsigned)sizeof(T);
+                    T s0 = T(0), s1 = T(0);
+#pragma unroll
+                    for (int e = 0; e < 16; e += 2) {
+                        T x0, x1, x2, x3, t0, t1, t2, t3;
+                        ts_lds2(xj + e * (unsigned)sizeof(T), x0, x1);
+                        ts_lds2(xj + (16 + e) * (unsigned)sizeof(T), x2, x3);
+                        ts_lds(tj + e * (unsigned)sizeof(T), t0);
+                        ts_lds(tj + (e + 1) * (unsigned)sizeof(T), t1);
+                        ts_lds(tj + (16 + e) * (unsigned)sizeof(T), t2);
+                        ts_lds(tj + (17 + e) * (unsigned)sizeof(T), t3);
+                        s0 = fma(t0, x0, s0);
+                        s1 = fma(t2, x2, s1);
+                        s0 = fma(t1, x1, s0);
+                        s1 = fma(t3, x3, s1);
+                    }
+                    y -= s0;
+                    y -= s1;
+                }
+                if (m == j && r < rows) {  // published beside the next warp's work
+                    st_stamped(slot + 2 * (r * BS_MAXR + q), P.epoch, (double)y);
+                    P.x[(size_t)(r0 + r) * P.ldx + q] = y;
                 }
             }
-            unsigned long long *slot = P.xslots + (size_t)r0 * (2 * BS_MAXR);
-            T *X = xs + buf * XB;
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                const int r = 32 * m + lane;
-                if (r < rows) st_stamped(slot + 2 * (r * BS_MAXR + warp), P.epoch, (double)y[m]);
-                X[xi(r, warp)] = r < rows ? y[m] : T(0);
-            }
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                const int r = 32 * m + lane;
-                if (r < rows) P.x[(size_t)(r0 + r) * P.ldx + warp] = y[m];
-            }
-        } else if (warp < NR) {
-            for (int r = lane; r < TS_B; r += 32) xs[buf * XB + xi(r, warp)] = T(0);
         }
         __syncthreads();
         if (k + 1 < n_own) prefetch_diag(k + 1);
     };
 
-    // this thread's row of owned block k in source p_src's tile
-    const int tr = tid >> 2, part = tid & 3;
-    auto tile_row = [&](int k, int p_src) -> int {
-        const int p = cta + k * G, r = r0_of(p) + tr;
-        if (tr >= rows_of(p)) return -1;
-        if (!LOWER || panel_of(p) == panel_of(p_src)) return r;
-        return __ldg(P.rows + (size_t)(panel_of(p_src) + 1) * P.n + r);  // its position after the source's panel
+    // The thread's part of a tile.  CUDA cores: row tid / 4, column pairs
+    // 8 j + 2 (tid % 4), of which the four threads of a row read 64 (float: 32)
+    // contiguous bytes per load.  Tensor pipe: the A fragments of rows
+    // 16 (warp % 8) + g, + 8 and columns 64 (warp / 8) + 8 j + {2 t, 2 t + 1}
+    // (the trailing update's permuted k), or, EXACT inside a panel, {t, t + 4}.
+    const int g = lane >> 2, t = lane & 3;
+    const int tr0 = MMA ? 16 * (warp & 7) + g : tid >> 2, half = warp >> 3;
+    constexpr int NROW = MMA ? 2 : 1;  // rows tr0, tr0 + 8
+    auto tile_rows = [&](int k, int p_src, int (&row)[NROW]) {
+        const int p = cta + k * G;
+#pragma unroll
+        for (int h = 0; h < NROW; h++) {
+            const int r = r0_of(p) + tr0 + 8 * h;
+            if (tr0 + 8 * h >= rows_of(p))
+                row[h] = -1;
+            else if (!LOWER || panel_of(p) == panel_of(p_src))
+                row[h] = r;
+            else
+                row[h] = __ldg(P.rows + (size_t)(panel_of(p_src) + 1) * P.n + r);  // its position after the source's panel
+        }
     };
-    // the thread's 32 columns of the tile's row as v (zero outside): column
-    // pairs 8 j + 2 part, 8 j + 2 part + 1 (j = 0..15), of which the four
-    // threads of a row read 64 (float: 32) contiguous bytes per load; or
-    // (EXACT) columns 32 part .. 32 part + 31
     const bool vec = ((reinterpret_cast<uintptr_t>(P.a) & (2 * sizeof(T) - 1)) == 0) && ((P.ld & 1) == 0) &&
                      (!LOWER || (P.nb & 1) == 0);
-    constexpr int CJ = EXACT ? 2 : 8, CP = EXACT ? 32 : 2;  // column of pair j of part: CJ j + CP part
-    auto load_tile = [&](int row, int p_src, T (&v)[TS_E]) {
+    auto load_tile = [&](int k, const int (&row)[NROW], int p_src, T (&v)[TS_E]) {
         const int c0 = r0_of(p_src), cols = rows_of(p_src);
-        if (row >= 0) {
-            const T *u = P.a + (size_t)row * P.ld + c0 + CP * part;
-            if (vec && cols == TS_B) {
+        const bool natural = EXACT && panel_of(cta + k * G) == panel_of(p_src);
 #pragma unroll
-                for (int j = 0; j < TS_E / 2; j++) ts_ld2(u + CJ * j, v[2 * j], v[2 * j + 1]);
-            } else {
+        for (int h = 0; h < NROW; h++) {
+            const int first = MMA ? 64 * half + (natural ? t : 2 * t) : 2 * (tid & 3);
+            const int second = natural ? 4 : 1;
+            const T *u = P.a + (size_t)max(row[h], 0) * P.ld + c0 + first;
 #pragma unroll
-                for (int j = 0; j < TS_E / 2; j++) {
-                    const int col = CJ * j + CP * part;
-                    v[2 * j] = col < cols ? __ldg(u + CJ * j) : T(0);
-                    v[2 * j + 1] = col + 1 < cols ? __ldg(u + CJ * j + 1) : T(0);
+            for (int j = 0; j < TS_E / 2 / NROW; j++) {
+                T &v0 = v[2 * (j * NROW + h)], &v1 = v[2 * (j * NROW + h) + 1];
+                v0 = v1 = T(0);
+                if (row[h] >= 0) {
+                    if (vec && !natural && cols == TS_B) {
+                        ts_ld2(u + 8 * j, v0, v1);
+                    } else {
+                        const int col = first + 8 * j;
+                        if (col < cols) v0 = __ldg(u + 8 * j);
+                        if (col + second < cols) v1 = __ldg(u + 8 * j + second);
+                    }
                 }
             }
-        } else {
-#pragma unroll
-            for (int e = 0; e < TS_E; e++) v[e] = T(0);
         }
     };
     // acc[k] -= tile * X; the first source of the block's own panel finds it
     // updated by all earlier panels and scales it by 1/pivot before
     auto apply_tile = [&](int k, int p_src, const T (&v)[TS_E], const T *X) {
         const int p = cta + k * G;
-        const bool own = LOWER && panel_of(p_src) == panel_of(p), live = tr < rows_of(p);
-        T *o = acc + ((size_t)k * TS_B + tr) * NR;
-        if constexpr (EXACT) {
-            if (!own) {
-                // the chain: right-hand side q is in part `part` at step q + part
-                T a = T(0);
-#pragma unroll 1
-                for (int step = 0; step < NR + 3; step++) {
-                    const int q = step - part;
-                    const T in = __shfl_up_sync(0xffffffffu, a, 1);
-                    const bool on = q >= 0 && q < NR;
-                    const int qc = on ? q : 0;
-                    a = part == 0 ? o[qc] : in;
-                    const T *xq = X + xi(32 * part, qc);
+        const bool own = LOWER && panel_of(p_src) == panel_of(p);
+        const bool scale = own && p_src % P.bpp == 0;
+        T *A = acc + (size_t)k * TS_B * NR;
+        if constexpr (MMA) {
+            double c[4];
+            double *o0 = A + tr0 * NR + 2 * t, *o1 = o0 + 8 * NR;  // rows tr0, tr0 + 8, right-hand sides 2t, 2t + 1
+            const double *xg = X + g * TS_XQ + 64 * half;           // B: k by 8 j + ..., column g
+            auto get = [&]() {
+                c[0] = o0[0];
+                c[1] = o0[1];
+                c[2] = o1[0];
+                c[3] = o1[1];
+            };
+            auto put = [&]() {
+                o0[0] = c[0];
+                o0[1] = c[1];
+                o1[0] = c[2];
+                o1[1] = c[3];
+            };
+            auto products = [&]() {  // c -= tile half * X
 #pragma unroll
-                    for (int g = 0; g < TS_E; g += 8) {  // the trailing update's order within 8 columns
-#pragma unroll
-                        for (int e = 0; e < 8; e += 2) a = fma(-v[g + e], xq[g + e], a);
-#pragma unroll
-                        for (int e = 1; e < 8; e += 2) a = fma(-v[g + e], xq[g + e], a);
-                    }
-                    if (part == 3 && on && live) o[q] = a;
+                for (int j = 0; j < 8; j++) {
+                    const double2 x = *reinterpret_cast<const double2 *>(xg + 8 * j + 2 * t);
+                    ts_mma(c, v[4 * j], v[4 * j + 2], v[4 * j + 1], v[4 * j + 3], -x.x, -x.y);
                 }
-                return;
+            };
+            if constexpr (!EXACT) {
+                c[0] = c[1] = c[2] = c[3] = 0.0;
+                products();
+                double *q0 = part_sum + tr0 * NR + 2 * t, *q1 = q0 + 8 * NR;
+                if (half == 1) {
+                    q0[0] = c[0];
+                    q0[1] = c[1];
+                    q1[0] = c[2];
+                    q1[1] = c[3];
+                }
+                __syncthreads();
+                if (half == 0) {
+                    o0[0] += c[0] + q0[0];
+                    o0[1] += c[1] + q0[1];
+                    o1[0] += c[2] + q1[0];
+                    o1[1] += c[3] + q1[1];
+                }
+                __syncthreads();  // part_sum is free again
+            } else if (!own) {
+                if (half == 0) {
+                    get();
+                    products();
+                    put();
+                }
+                __syncthreads();
+                if (half == 1) {
+                    get();
+                    products();
+                    put();
+                }
+            } else {
+                double s[4][4];  // 16 columns each
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    s[b][0] = s[b][1] = s[b][2] = s[b][3] = 0.0;
+#pragma unroll
+                    for (int j = 2 * b; j < 2 * b + 2; j++)
+                        ts_mma(s[b], v[4 * j], v[4 * j + 2], v[4 * j + 1], v[4 * j + 3], xg[8 * j + t],
+                               xg[8 * j + t + 4]);
+                }
+                if (half == 0) {
+                    get();
+                    if (scale) {
+                        const double d0 = sdinv[k * TS_B + tr0], d1 = sdinv[k * TS_B + tr0 + 8];
+                        c[0] *= d0;
+                        c[1] *= d0;
+                        c[2] *= d1;
+                        c[3] *= d1;
+                    }
+#pragma unroll
+                    for (int b = 0; b < 4; b++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) c[e] -= s[b][e];
+                    put();
+                }
+                __syncthreads();
+                if (half == 1) {
+                    get();
+#pragma unroll
+                    for (int b = 0; b < 4; b++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) c[e] -= s[b][e];
+                    put();
+                }
             }
-            const bool scale = p_src % P.bpp == 0;
-            const T d = scale ? sdinv[k * TS_B + tr] : T(1);
-#pragma unroll 1
+        } else {
+            T s[NR];
+#pragma unroll
             for (int q = 0; q < NR; q++) {
-                const T *xq = X + xi(32 * part, q);
+                const T *xq = X + q * TS_XQ + 2 * (tid & 3);
                 T s0 = T(0), s1 = T(0);
 #pragma unroll
-                for (int e = 0; e < 16; e++) {
-                    s0 = fma(v[e], xq[e], s0);
-                    s1 = fma(v[16 + e], xq[16 + e], s1);
+                for (int j = 0; j < TS_E / 2; j++) {
+                    s0 = fma(v[2 * j], xq[8 * j], s0);
+                    s1 = fma(v[2 * j + 1], xq[8 * j + 1], s1);
                 }
-                T a = o[q];
-                if (scale) a *= d;
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    a -= __shfl_sync(0xffffffffu, s0, (lane & ~3) + e);
-                    a -= __shfl_sync(0xffffffffu, s1, (lane & ~3) + e);
-                }
-                __syncwarp();
-                if (part == 0 && live) o[q] = a;
+                s[q] = s0 + s1;
+                s[q] += __shfl_xor_sync(0xffffffffu, s[q], 1);
+                s[q] += __shfl_xor_sync(0xffffffffu, s[q], 2);
             }
-            return;
-        }
-        T s[NR];
+            if ((tid & 3) == 0 && tr0 < rows_of(p)) {
+                const T d = scale ? sdinv[k * TS_B + tr0] : T(1);
 #pragma unroll
-        for (int q = 0; q < NR; q++) s[q] = T(0);
-#pragma unroll
-        for (int e = 0; e < TS_E; e++) {
-            const T *xr = X + xi(8 * (e >> 1) + 2 * part + (e & 1), 0);
-#pragma unroll
-            for (int q = 0; q < NR; q++) s[q] += v[e] * xr[q];
-        }
-#pragma unroll
-        for (int q = 0; q < NR; q++) {
-            s[q] += __shfl_xor_sync(0xffffffffu, s[q], 1);
-            s[q] += __shfl_xor_sync(0xffffffffu, s[q], 2);
-        }
-        if (part == 0 && live) {
-            const bool scale = own && p_src % P.bpp == 0;
-            const T d = LOWER && scale ? sdinv[k * TS_B + tr] : T(1);
-#pragma unroll
-            for (int q = 0; q < NR; q++) o[q] = (scale ? o[q] * d : o[q]) - s[q];
+                for (int q = 0; q < NR; q++) {
+                    T &o = A[tr0 * NR + q];
+                    o = (scale ? o * d : o) - s[q];
+                }
+            }
         }
     };
 
@@ -354,15 +464,18 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParam
         next = 1;
     }
     const unsigned long long t0 = globaltimer_ns();
-    int row = next < n_own ? tile_row(next, 0) : -1;
+    int row[NROW];
+#pragma unroll
+    for (int h = 0; h < NROW; h++) row[h] = -1;
+    if (next < n_own) tile_rows(next, 0, row);
     for (int p_src = 0; p_src < nblk; p_src++) {
         const int buf = p_src & 1;
         T *X = xs + buf * XB;
         const int k_first = next;
         T v[TS_E];
         if (k_first < n_own) {
-            load_tile(row, p_src, v);
-            if (p_src + 1 < nblk) row = tile_row(k_first, p_src + 1);
+            load_tile(k_first, row, p_src, v);
+            if (p_src + 1 < nblk) tile_rows(k_first, p_src + 1, row);
         }
         if (p_src % G != cta && k_first < n_own) {
             // the source block's x from its slots: each thread re-loads its
@@ -375,11 +488,11 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParam
 #pragma unroll
             for (int u = 0; u < EPT; u++) {
                 const int e = tid + u * TS_THREADS, r = e / NR, q = e % NR;
-                if (e >= TS_B * NR) continue;
-                if (r < rows && q < P.nr)
+                if (e >= TS_B * NR || q >= P.nr) continue;
+                if (r < rows)
                     todo |= 1u << u;
                 else
-                    X[xi(r, q)] = T(0);
+                    X[q * TS_XQ + r] = T(0);
             }
             for (unsigned round = 1;; round++) {
 #pragma unroll
@@ -389,7 +502,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParam
                     unsigned long long hi, lo;
                     ld_pair(slot + 2 * (r * BS_MAXR + q), hi, lo);
                     if (stamped(hi, P.epoch) && stamped(lo, P.epoch)) {
-                        X[xi(r, q)] = (T)unstamp(hi, lo);
+                        X[q * TS_XQ + r] = (T)unstamp(hi, lo);
                         todo &= ~(1u << u);
                     }
                 }
@@ -408,11 +521,13 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParam
                 __syncthreads();
                 solve(k_first, buf ^ 1);
                 next = k_first + 1;
-                if (next < n_own && p_src + 1 < nblk) row = tile_row(next, p_src + 1);
+                if (next < n_own && p_src + 1 < nblk) tile_rows(next, p_src + 1, row);
             }
         }
         for (int k = k_first + 1; k < n_own; k++) {
-            load_tile(tile_row(k, p_src), p_src, v);
+            int rk[NROW];
+            tile_rows(k, p_src, rk);
+            load_tile(k, rk, p_src, v);
             apply_tile(k, p_src, v, X);
         }
         __syncthreads();  // X (this buffer) is overwritten two sources later
@@ -428,7 +543,9 @@ static cudaError_t ts_launch(TriParams<T> P, cudaStream_t st, bool *used)
     if (e != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     const int G = P.nblk < sms ? P.nblk : sms, own = (P.nblk + G - 1) / G;
-    const size_t smem = ((size_t)TS_B * TS_TLD + 2 * TS_XBUF * NR + (size_t)own * TS_B * (NR + (LOWER ? 1 : 0))) * sizeof(T);
+    const size_t smem = ((size_t)TS_B * TS_TLD + 2 * TS_XQ * NR + (NR == 8 && !LOWER ? TS_B * NR : 0) +
+                         (size_t)own * TS_B * (NR + (LOWER ? 1 : 0))) *
+                        sizeof(T);
     if (smem > 220 * 1024) return cudaSuccess;  // too many blocks per CTA: the caller's other way
     auto kern = tri_solve_kernel<T, LOWER, NR>;
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)) != cudaSuccess) return e;
@@ -439,7 +556,14 @@ static cudaError_t ts_launch(TriParams<T> P, cudaStream_t st, bool *used)
     return e;
 }
 
-// up to BS_MAXR right-hand sides, padded to the next of 1, 2, 4, 8
+// right-hand sides one launch takes: FP32 solves, of one vector each, stay on
+// the CUDA cores
+template <typename T>
+static constexpr int ts_maxr()
+{
+    return sizeof(T) == 8 ? BS_MAXR : 1;
+}
+
 template <typename T, bool LOWER>
 static cudaError_t ts_any(TriParams<T> P, const BsBuffers &bs, cudaStream_t st, bool *used)
 {
@@ -449,10 +573,7 @@ static cudaError_t ts_any(TriParams<T> P, const BsBuffers &bs, cudaStream_t st, 
     P.status = bs.status;
     P.epoch = ++*bs.epoch;
     if (P.epoch == 0) P.epoch = ++*bs.epoch;
-    if (P.nr == 1) return ts_launch<T, LOWER, 1>(P, st, used);
-    if (P.nr == 2) return ts_launch<T, LOWER, 2>(P, st, used);
-    if (P.nr <= 4) return ts_launch<T, LOWER, 4>(P, st, used);
-    return ts_launch<T, LOWER, 8>(P, st, used);
+    return ts_launch<T, LOWER, ts_maxr<T>()>(P, st, used);
 }
 
 template <typename T>
@@ -460,7 +581,7 @@ static cudaError_t upper_t(const T *a, long ld, int n, int nrhs, const T *y, lon
                            const BsBuffers &bs, cudaStream_t st, bool *used)
 {
     *used = false;
-    for (int c0 = 0; c0 < nrhs; c0 += BS_MAXR) {
+    for (int c0 = 0; c0 < nrhs; c0 += ts_maxr<T>()) {
         TriParams<T> P{};
         P.a = a;
         P.ld = ld;
@@ -472,7 +593,7 @@ static cudaError_t upper_t(const T *a, long ld, int n, int nrhs, const T *y, lon
         P.ldy = ldy;
         P.x = x + c0;
         P.ldx = ldx;
-        P.nr = nrhs - c0 < BS_MAXR ? nrhs - c0 : BS_MAXR;
+        P.nr = nrhs - c0 < ts_maxr<T>() ? nrhs - c0 : ts_maxr<T>();
         const cudaError_t e = ts_any<T, false>(P, bs, st, used);
         if (e != cudaSuccess || !*used) return e;  // the first chunk decides: all have the same blocks
     }
@@ -496,7 +617,7 @@ static cudaError_t lower_t(const T *a, long ld, int n, int nb, const int *rows, 
                            int nrhs, T *y, long ldy, const BsBuffers &bs, cudaStream_t st, bool *used)
 {
     *used = false;
-    if (nrhs > BS_MAXR) return cudaErrorInvalidValue;
+    if (nrhs > ts_maxr<T>()) return cudaErrorInvalidValue;
     TriParams<T> P{};
     P.a = a;
     P.ld = ld;
