@@ -13,28 +13,33 @@
 // of a CTA spends on it.  Over the whole grid that chain costs four trips
 // through L2 per column (kernels_leaf.cu: 3.6-4.6 us); inside a cluster it is
 // two CTA barriers and one trip through distributed shared memory.  So:
-//  * S neighbouring lanes hold R whole rows in registers, a row's columns dealt
-//    to them in turn; lane q of the S also keeps the book of rows q, q + S, ...
-//    of the R (their position, their part in the pivot search).  One lane per
-//    row would read the pivot row from shared memory R times as often, one
-//    book per lane and row would repeat its work S times.  256 threads, since
-//    whatever all warps do costs issue slots per warp.
-//  * no row ever moves: an exchange c <-> p is two rows changing their
-//    positions (`pos`), and a row is written back to its last one at the end.
-//  * the registers rotate: after S columns the rows move down by one register,
-//    so the columns are one rolled loop (its current column always in register
-//    0), small enough for the instruction cache (a body unrolled over the S
-//    columns and four widths measured 1.75 us a column, most of it fetch).
-//    The multiplier l goes to the row's shared-memory slot, which is stored to
-//    the matrix at the end.
+//  * the slab lives in the CTAs' shared memory and is factored in blocks of 8
+//    columns, each thread holding the 8 columns of its RT rows in registers.
+//    The registers rotate (eliminating a column writes r[j+1] - l u[j+1] into
+//    r[j]), so the 8 columns are one rolled loop, small enough for the
+//    instruction cache.  A pivot decision then concerns 8 columns: its row is
+//    written by one lane in 5 shared stores and travels as 5 pieces of 16
+//    bytes.  (Rows of all 64 columns in registers, searched, scaled, sent and
+//    updated whole at every column, took 1.14 us a column on one CTA and 1.66
+//    on 16.)
+//  * no row ever moves: each carries its current position in the matrix
+//    (`pos`), an exchange c <-> p is two rows changing their positions, and a
+//    row is written back to its last one at the end.
 //  * a warp's candidate is found with redux.sync on the bits of |a| (the upper
 //    word decides except in ties), the CTA's from the warps' after one
-//    barrier; its owner puts the row, already scaled by 1/pivot, into shared
-//    memory, from where after a second barrier all warps send it to every CTA
-//    of the cluster with st.async, which completes an mbarrier there.  Every
-//    warp then picks the winner from the CTAs' candidates by itself.  (Sending
-//    the candidates' keys first and the winner's row alone in a second trip
-//    measured 1000-1300 cycles a column against 750-1100 for the one trip.)
+//    barrier; its owner puts the row, scaled by 1/pivot, into shared memory,
+//    from where after a second barrier it goes to every CTA of the cluster with
+//    st.async, which completes an mbarrier there.  Every warp then picks the
+//    winner from the CTAs' candidates by itself.  (Sending the candidates' keys
+//    first and the winner's row alone in a second trip measured 1000-1300
+//    cycles a column against 750-1100 for the one trip.)
+//  * the winner's CTA sends the rest of the row, unchanged since the block
+//    began, to every CTA on a second mbarrier, beside the next columns.  After
+//    the 8 columns every CTA finishes the 8 pivot rows right of the block by
+//    itself (one thread per column, the same multiply-adds in the same order)
+//    and subtracts their products from its rows: FP64 on the tensor pipe
+//    (mma.sync m16n8k8, which adds its products in k order), FP32 on the CUDA
+//    cores.
 // Messages are double-buffered by column parity: a CTA can be one column ahead
 // of another at most, since it needs that CTA's message of a column to leave
 // it, and a buffer's readers have passed the next column's CTA barriers before
@@ -62,19 +67,28 @@ struct CLeafParams {
     int withhold;
 };
 
-template <typename T, int W, int S, int R, int TPB>
+constexpr int CL_TPB = 256, CL_NW = CL_TPB / 32;  // threads with rows
+constexpr int CL_HELP = 128;  // helpers: store and send the decided rows beside the next column's search
+constexpr int CL_ALL = CL_TPB + CL_HELP;
+constexpr int CL_B = 8;      // columns of a block
+constexpr int CL_MAXC = 16;  // CTAs of a cluster
+
+template <typename T, int W, int RT>
 struct CLeafCfg {
-    static constexpr int NW = TPB / 32;
     static constexpr int VEC = 16 / (int)sizeof(T);
-    static constexpr int PITCH = W + VEC;     // a slot's 16-byte accesses by consecutive rows hit distinct banks
-    static constexpr int ROWS = R * TPB / S;  // rows a CTA holds
-    static constexpr int ROWB = (W + S * VEC) * (int)sizeof(T);  // a travelling row: each lane's part and 16 bytes of padding
-    static constexpr int MSG = 16 + ROWB;                        // header (key, position), then the row
-    static constexpr int MAXC = 16;
+    static constexpr int PITCH = W + VEC;      // 16-byte accesses of consecutive rows fall on distinct banks
+    static constexpr int ROWS = RT * CL_TPB;   // rows a CTA holds
+    static constexpr int MSG = 16 + CL_B * (int)sizeof(T);  // header (key, position, row), the row's 8 columns
+    static constexpr int PIECES = MSG / 16;
+    static constexpr int UP = W + 4;           // pitch of the finished pivot rows: B fragments on distinct banks
+    static constexpr int XP = W + VEC;         // pitch of the received pivot rows
     static constexpr size_t O_SLAB = 0;
-    static constexpr size_t O_MSG = O_SLAB + (size_t)ROWS * PITCH * sizeof(T);
-    static constexpr size_t O_POS = O_MSG + (size_t)2 * MAXC * MSG;
+    static constexpr size_t O_U = O_SLAB + (size_t)ROWS * PITCH * sizeof(T);
+    static constexpr size_t O_X = O_U + (size_t)CL_B * UP * sizeof(T);
+    static constexpr size_t O_MSG = O_X + (size_t)CL_B * XP * sizeof(T);
+    static constexpr size_t O_POS = O_MSG + (size_t)2 * CL_MAXC * MSG;
     static constexpr size_t SMEM = O_POS + (size_t)ROWS * sizeof(int);
+    static_assert(O_X % 16 == 0 && O_MSG % 16 == 0 && MSG % 16 == 0, "16-byte pieces");
 };
 
 __device__ __forceinline__ unsigned cl_smem(const void *p)
@@ -83,16 +97,21 @@ __device__ __forceinline__ unsigned cl_smem(const void *p)
 }
 
 // Pivot candidates order as (key, then lower position): key 0 = not a
-// candidate, 1 = row c when nothing else is left (a column of NaNs keeps its
-// row), else the bits of |v| + 2 -- for float in the upper word.  A thread's
-// best of its rows is kept as a value: -2 for none, -1 for such a row c.
-__device__ __forceinline__ unsigned long long cl_key(double best)
+// candidate, 1 = row c holding a NaN (taken when nothing else is left: such a
+// column keeps its row), else the bits of |v| with 2 added to the upper word.
+// A float's key is its upper word alone.  (Integer tests: a 64-bit floating
+// comparison costs the chain 20 cycles.)
+__device__ __forceinline__ unsigned long long cl_key(double v, bool act, bool at_c)
 {
-    return best >= 0.0 ? (unsigned long long)__double_as_longlong(best) + 2ull : (best > -1.5 ? 1ull : 0ull);
+    const unsigned hi = (unsigned)__double2hiint(v) & 0x7fffffffu, lo = (unsigned)__double2loint(v);
+    const bool nan = (hi > 0x7ff00000u) | ((hi == 0x7ff00000u) & (lo != 0u));
+    const unsigned kh = act ? (nan ? (unsigned)at_c : hi + 2u) : 0u, kl = act & !nan ? lo : 0u;
+    return (unsigned long long)kh << 32 | kl;
 }
-__device__ __forceinline__ unsigned long long cl_key(float best)
+__device__ __forceinline__ unsigned long long cl_key(float v, bool act, bool at_c)
 {
-    return (unsigned long long)(best >= 0.f ? __float_as_uint(best) + 2u : (best > -1.5f ? 1u : 0u)) << 32;
+    const unsigned b = __float_as_uint(v) & 0x7fffffffu;
+    return (unsigned long long)(act ? (b > 0x7f800000u ? (unsigned)at_c : b + 2u) : 0u) << 32;
 }
 __device__ __forceinline__ bool cl_zero(double v) { return ((unsigned long long)__double_as_longlong(v) << 1) == 0; }
 __device__ __forceinline__ bool cl_zero(float v) { return (__float_as_uint(v) << 1) == 0; }
@@ -176,212 +195,41 @@ __device__ __forceinline__ void cl_stu(unsigned p, unsigned long long a, unsigne
     asm volatile("st.shared.v2.u64 [%0], {%1, %2};" ::"r"(p), "l"(a), "l"(b) : "memory");
 }
 
-// One CTA's part in the columns of the leaf
-template <typename T, int W, int S, int R, int TPB>
-struct CLeaf {
-    using C = CLeafCfg<T, W, S, R, TPB>;
-    static constexpr int NW = C::NW, VEC = C::VEC, PITCH = C::PITCH, MSG = C::MSG;
-    static constexpr int WL = W / S;         // columns of a row per lane
-    static constexpr int M = R / S;          // rows a lane keeps the book of
-    static constexpr int LSTR = WL + VEC;    // elements between the lanes' parts of a travelling row
-    static constexpr int PPL = WL / VEC;     // 16-byte pieces per lane's part
-    static_assert(R % S == 0 && W % S == 0 && WL % VEC == 0, "rows and columns dealt evenly");
-    struct Shared {
-        alignas(16) unsigned long long cand[NW][2];  // the warps' candidates: key, position
-        int fail;             // set in a column's wait, read after the next column's first barrier
-        unsigned long long bar[2];
-        T d[W], inv[W];  // the pivots, at the end their reciprocals
-        int piv[W];
-        alignas(16) unsigned char out[MSG];       // the CTA's candidate of the column
-        alignas(16) unsigned char none[C::ROWB];  // zeros: what a zero pivot's column subtracts
-    };
-    struct Rows {
-        T r[R][WL];  // row k, register i of lane q: column i S + q of what is left
-        T ls[M];     // row m S + q: the multiplier the reference's pivot searches look at
-        int pos[M];  // its current position (rows of the view); -1: no row
-    };
+__device__ __forceinline__ void cl_mma(double (&c)[4], double a0, double a1, double a2, double a3, double b0, double b1)
+{
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};\n"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
+}
 
-    // Every column of the leaf; false when a wait gave up.
-    static __device__ __forceinline__ bool columns(const CLeafParams<T> &P, Shared &sh, unsigned char *dyn, Rows &x)
-    {
-        const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane % S;
-        const int CL = gridDim.x, rank = blockIdx.x, w = P.w;
-        constexpr unsigned ES = sizeof(T);
-        const unsigned slot = cl_smem(dyn + C::O_SLAB) + tid * PITCH * ES;  // of this lane's first row
-        const unsigned msg = cl_smem(dyn + C::O_MSG), out = cl_smem(sh.out), none = cl_smem(sh.none);
-        const unsigned cands = cl_smem(&sh.cand[0][0]), failed = cl_smem(&sh.fail);
-        // this thread's share of the sends: pieces p0, p0 + tpd, ... to CTA `to`
-        const int tpd = TPB / CL, to = tid / tpd, p0 = tid - to * tpd;
-        const unsigned bar0 = cl_smem(&sh.bar[0]);
-        unsigned rmsg, rbar;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rmsg) : "r"(msg + rank * MSG), "r"(to));
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbar) : "r"(bar0), "r"(to));
+__device__ __forceinline__ unsigned cl_mapa(unsigned p, int rank)
+{
+    unsigned d;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(p), "r"(rank));
+    return d;
+}
 
-#pragma unroll 1
-        for (int ip = 0; ip < w; ip++) {
-            const int c = P.c0 + ip, par = ip & 1, s = ip % S, left = w - ip + s;  // columns from the group's first on
-            const bool use_ls = ip > 0 && ((P.mode == PIVOT_REF && ((c + P.goff) & 1)) ||  // lu2tlib.c:1052
-                                           P.mode == PIVOT_REF_FIRST);
-            // the column to all lanes of its rows (they are the multipliers)
-            T l[R], lm[M];
-#pragma unroll
-            for (int k = 0; k < R; k++) l[k] = S == 1 ? x.r[k][0] : __shfl_sync(0xffffffffu, x.r[k][0], lane - q + s);
-            // this thread's candidate, the warp's, the CTA's
-            T best = T(-2), kd = T(1);
-            int kp = INT_MAX, kr = 0;
-#pragma unroll
-            for (int m = 0; m < M; m++) {
-                lm[m] = l[m * S];
-#pragma unroll
-                for (int e = 1; e < S; e++) lm[m] = q == e ? l[m * S + e] : lm[m];
-                T v = lm[m];
-                if (use_ls) v = x.ls[m];
-                v = fabs(v);
-                const int pm = x.pos[m];
-                const bool act = pm >= c;
-                bool take = act & ((v > best) | ((v == best) & (pm < kp)));
-                const bool keep = act & (pm == c) & (best < T(-1)) & !take;
-                best = take ? v : (keep ? T(-1) : best);
-                take |= keep;
-                kp = take ? pm : kp;
-                kr = take ? m * S + q : kr;
-                kd = take ? lm[m] : kd;
-            }
-            const unsigned long long key = cl_key(best);
-            const int wl = cl_winner(key, kp, lane);
-            if (lane == wl) cl_stu(cands + 16 * warp, key, (unsigned)kp);
-            __syncthreads();
-            unsigned long long ck = 0ull, cp = INT_MAX;
-            if (lane < NW) cl_ldu(cands + 16 * lane, ck, cp);
-            if (cl_ldi(failed)) return false;
-            if (warp == cl_winner(ck, (int)cp, lane)) {
-                T inv = cl_zero(kd) ? T(1) : T(1) / kd;
-                inv = __shfl_sync(0xffffffffu, inv, wl);
-                kr = __shfl_sync(0xffffffffu, kr, wl);
-                if (lane / S == wl / S) {
-                    const unsigned dst = out + 16 + q * LSTR * ES;
-#pragma unroll
-                    for (int k = 0; k < R; k++)
-                        if (kr == k) {
-#pragma unroll
-                            for (int j = 0; j < WL; j += VEC)
-                                if (j * S < left) {
-                                    T v[VEC];
-#pragma unroll
-                                    for (int e = 0; e < VEC; e++)
-                                        v[e] = j + e == 0 && q == s ? x.r[k][0] : x.r[k][j + e] * inv;
-                                    cl_st16(dst + j * ES, v);
-                                }
-                        }
-                }
-                if (lane == wl) cl_stu(out, key, (unsigned)kp);
-            }
-            __syncthreads();
-            unsigned bst = out;
-            if (CL > 1) {
-                const int pieces = 1 + S * min(PPL, (left - 1) / (S * VEC) + 1);
-                if (tid == 0)
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar0 + 8 * par),
-                                 "r"(CL * 16 * pieces)
-                                 : "memory");
-                if (rank != P.withhold)
-#pragma unroll 1
-                    for (int i = p0; i < pieces; i += tpd) {
-                        // header, then register pieces by lane
-                        const unsigned at = i == 0 ? 0 : 16 + ((i - 1) % S) * LSTR * ES + ((i - 1) / S) * 16;
-                        unsigned long long v0, v1;
-                        cl_ldu(out + at, v0, v1);
-                        asm volatile(
-                            "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(
-                                rmsg + par * C::MAXC * MSG + at),
-                            "l"(v0), "l"(v1), "r"(rbar + 8 * par)
-                            : "memory");
-                    }
-                // every CTA's candidate of this column
-                if (!arrived(P, bar0 + 8 * par, (unsigned)(ip >> 1) & 1u)) sh.fail = 1;  // leaves at the next barrier
-                __syncwarp();
-                const unsigned m0 = msg + par * C::MAXC * MSG;
-                ck = 0ull;
-                cp = INT_MAX;
-                if (lane < CL) cl_ldu(m0 + lane * MSG, ck, cp);
-                bst = m0 + cl_winner(ck, (int)cp, lane) * MSG;
-            }
-            const int p = cl_ldi(bst + 8);
-            const unsigned u = bst + 16;
-            T d;
-            cl_ld1(u + s * LSTR * ES, d);
-            unsigned uq = u + q * LSTR * ES;
-            if (cl_zero(d)) {
-                uq = none;
-#pragma unroll
-                for (int k = 0; k < R; k++) l[k] = T(0);
-            }
-            // the pivot row's part of this lane
-            T v[WL];
-#pragma unroll
-            for (int j = 0; j < WL; j += VEC)
-                if (j * S < left) {
-                    T t[VEC];
-                    cl_ld16(uq + j * ES, t);
-#pragma unroll
-                    for (int e = 0; e < VEC; e++) v[j + e] = t[e];
-                }
-#pragma unroll
-            for (int m = 0; m < M; m++) {
-                const int pm = x.pos[m];
-                if (pm >= c && pm != p) cl_st1(slot + (m * TPB * PITCH + ip) * ES, lm[m]);
-                x.pos[m] = pm == p ? c : (pm == c ? p : pm);
-                if (P.mode == PIVOT_REF || ip == 0) x.ls[m] = lm[m];
-            }
-            // rank-1 update; rows that are done compute values nobody reads, as
-            // do lanes up to s in register 0.  After the last of S columns the
-            // rows move down by a register.
-            if (s != S - 1) {
-#pragma unroll
-                for (int j = 0; j < WL; j += VEC)
-                    if (j * S < left) {
-#pragma unroll
-                        for (int e = 0; e < VEC; e++)
-#pragma unroll
-                            for (int k = 0; k < R; k++) x.r[k][j + e] = cl_fnma(l[k], v[j + e], x.r[k][j + e]);
-                    }
-            } else {
-#pragma unroll
-                for (int j = 0; j < WL; j += VEC)
-                    if (j * S < left) {
-#pragma unroll
-                        for (int e = 0; e < VEC; e++)
-                            if (j + e > 0) {
-#pragma unroll
-                                for (int k = 0; k < R; k++) x.r[k][j + e - 1] = cl_fnma(l[k], v[j + e], x.r[k][j + e]);
-                            }
-                    }
-            }
-            // row c of the factors from column c on (the warps take turns)
-            if (warp == (ip & (NW - 1))) {
-                if (rank == 0) {
-                    T *dst = P.a + (size_t)c * P.ld + c - s;  // column c - s + j: part j % S, register j / S
-                    for (int j = s + lane; j < left; j += 32) {
-                        T t;
-                        cl_ld1(u + ((j % S) * LSTR + j / S) * ES, t);
-                        dst[j] = t;
-                    }
-                }
-                if (lane == 0) {
-                    sh.d[ip] = d;
-                    sh.piv[ip] = p;
-                }
-            }
-        }
-        return true;
-    }
+// 16 bytes to another CTA's shared memory, counted by its mbarrier
+__device__ __forceinline__ void cl_send(unsigned dst, unsigned long long a, unsigned long long b, unsigned bar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst), "l"(a),
+                 "l"(b), "r"(bar)
+                 : "memory");
+}
 
-    // bounded wait for a column's messages; records the error when it gives up
-    static __device__ __forceinline__ bool arrived(const CLeafParams<T> &P, unsigned bar, unsigned parity)
-    {
-        unsigned long long t0 = 0;
-#pragma unroll 1
-        for (unsigned spins = 1;; spins++) {
+__device__ __forceinline__ void cl_expect(unsigned bar, int bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+// bounded wait for an mbarrier's phase; records the error when it gives up
+__device__ __noinline__ bool cl_wait_slow(unsigned bar, unsigned parity, int *status, unsigned long long limit)
+{
+    const unsigned long long t0 = globaltimer_ns();
+    for (;;) {
+        for (int spins = 0; spins < 16; spins++) {
             unsigned ok;
             asm volatile(
                 "{\n\t.reg .pred P1;\n\t"
@@ -391,78 +239,415 @@ struct CLeaf {
                 : "r"(bar), "r"(parity)
                 : "memory");
             if (ok) return true;
-            if ((spins & 15u) == 0) {
-                const unsigned long long now = globaltimer_ns();
-                if (t0 == 0) t0 = now;
-                if (*(volatile int *)&P.status[1] != 0) return false;
-                if (now - t0 > P.wait_ns) {
-                    record_error(P.status, ERR_BARRIER_TIMEOUT, 1);
-                    return false;
-                }
+        }
+        if (*(volatile int *)&status[1] != 0) return false;
+        if (globaltimer_ns() - t0 > limit) {
+            record_error(status, ERR_BARRIER_TIMEOUT, 1);
+            return false;
+        }
+    }
+}
+__device__ __forceinline__ bool cl_wait(unsigned bar, unsigned parity, int *status, unsigned long long limit)
+{
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred P1;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P1, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, P1;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok || cl_wait_slow(bar, parity, status, limit);
+}
+
+template <typename T, int W>
+struct CLeafShared {
+    alignas(16) unsigned long long cand[CL_NW][2];  // the warps' candidates: key, position
+    alignas(16) unsigned char out[16 + CL_B * sizeof(T)];  // the CTA's candidate of the column
+    unsigned long long bar[3];  // messages of even and odd columns; the pivot rows of a block
+    int fail;                   // set in a wait, read after the next barrier
+    T d[W], inv[W];             // the pivots, their reciprocals
+    int piv[W];
+    unsigned row[CL_B];         // the block's pivot rows: shared address of column 0 (own slab, or received)
+};
+
+// Rows blk + 8 .. of the block's 8 pivot rows, finished; then their products
+// off the CTA's rows.  c1 = the position after the block, rem columns right of it.
+template <int W, int RT>
+__device__ __forceinline__ void cl_update(const CLeafCfg<double, W, RT> *, unsigned slab, unsigned ub, unsigned spos,
+                                          const double (&dz)[2], int blk, int rem, int c1)
+{
+    using C = CLeafCfg<double, W, RT>;
+    // a warp's 32 RT rows as 2 RT tiles of 16: fragment row g is tile row pg,
+    // so that the rows a quarter-warp touches fall on distinct banks
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int pg = (g >> 1) + ((g & 1) << 2);
+    const unsigned r0 = slab + (warp * 32 * RT + pg) * C::PITCH * 8;
+    constexpr int MT = RT > 2 ? 4 : 2 * RT;  // tiles at a time
+#pragma unroll 1
+    for (int pass = 0; pass < 2 * RT / MT; pass++) {
+        const unsigned rp = r0 + pass * MT * 16 * C::PITCH * 8;
+        const int row0 = warp * 32 * RT + pass * MT * 16 + pg;
+        double a[MT][4];
+        unsigned live = 0;
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int row = 16 * m + 8 * h;
+                cl_ld1(rp + (row * C::PITCH + blk + t) * 8, a[m][h]);
+                cl_ld1(rp + (row * C::PITCH + blk + t + 4) * 8, a[m][2 + h]);
+                // -l, and nothing of a zero pivot's column
+                a[m][h] = dz[0] == 0.0 ? 0.0 : -a[m][h];
+                a[m][2 + h] = dz[1] == 0.0 ? 0.0 : -a[m][2 + h];
+                if (cl_ldi(spos + (row0 + row) * 4) >= c1) live |= 1u << (2 * m + h);  // done rows stay
+            }
+#pragma unroll 1
+        for (int n0 = 0; n0 < rem; n0 += 8) {
+            double b0, b1;
+            cl_ld1(ub + (t * C::UP + n0 + g) * 8, b0);
+            cl_ld1(ub + ((t + 4) * C::UP + n0 + g) * 8, b1);
+            double lo[MT][2], hi[MT][2];
+            const unsigned p = rp + (blk + CL_B + n0 + 2 * t) * 8;
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                cl_ld16(p + 16 * m * C::PITCH * 8, lo[m]);
+                cl_ld16(p + (16 * m + 8) * C::PITCH * 8, hi[m]);
+            }
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                double c[4] = {lo[m][0], lo[m][1], hi[m][0], hi[m][1]};
+                cl_mma(c, a[m][0], a[m][1], a[m][2], a[m][3], b0, b1);
+                lo[m][0] = c[0];
+                lo[m][1] = c[1];
+                hi[m][0] = c[2];
+                hi[m][1] = c[3];
+            }
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                if (live >> (2 * m) & 1) cl_st16(p + 16 * m * C::PITCH * 8, lo[m]);
+                if (live >> (2 * m + 1) & 1) cl_st16(p + (16 * m + 8) * C::PITCH * 8, hi[m]);
             }
         }
     }
-};
-
-template <typename T, int W, int S, int R, int TPB>
-__global__ void __launch_bounds__(TPB, 1) cluster_leaf_kernel(const CLeafParams<T> P)
+}
+template <int W, int RT>
+__device__ __forceinline__ void cl_update(const CLeafCfg<float, W, RT> *, unsigned slab, unsigned ub, unsigned spos,
+                                          const float (&dz)[8], int blk, int rem, int c1)
 {
-    using C = CLeafCfg<T, W, S, R, TPB>;
-    using L = CLeaf<T, W, S, R, TPB>;
-    constexpr int VEC = C::VEC, PITCH = C::PITCH;
+    using C = CLeafCfg<float, W, RT>;
+    // each thread its own rows, two at a time
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < RT; k += 2) {
+        float l[2][CL_B];
+        unsigned row[2];
+        bool live[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int lr = tid + (k + h) * CL_TPB;
+            row[h] = slab + (lr * C::PITCH + blk) * 4;
+            live[h] = cl_ldi(spos + lr * 4) >= c1;
+#pragma unroll
+            for (int j = 0; j < CL_B; j += 4) {
+                float v[4];
+                cl_ld16(row[h] + j * 4, v);
+#pragma unroll
+                for (int e = 0; e < 4; e++) l[h][j + e] = dz[j + e] == 0.f ? 0.f : v[e];
+            }
+        }
+#pragma unroll 1
+        for (int n0 = 0; n0 < rem; n0 += 4) {
+            float c[2][4];
+            cl_ld16(row[0] + (CL_B + n0) * 4, c[0]);
+            cl_ld16(row[1] + (CL_B + n0) * 4, c[1]);
+#pragma unroll
+            for (int j = 0; j < CL_B; j++) {
+                float u[4];
+                cl_ld16(ub + (j * C::UP + n0) * 4, u);
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) c[h][e] = cl_fnma(l[h][j], u[e], c[h][e]);
+            }
+            if (live[0]) cl_st16(row[0] + (CL_B + n0) * 4, c[0]);
+            if (live[1]) cl_st16(row[1] + (CL_B + n0) * 4, c[1]);
+        }
+    }
+}
+
+template <typename T, int W, int RT>
+__global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafParams<T> P)
+{
+    using C = CLeafCfg<T, W, RT>;
+    constexpr int VEC = C::VEC, PITCH = C::PITCH, MSG = C::MSG, PIECES = C::PIECES;
+    constexpr unsigned ES = sizeof(T);
     extern __shared__ __align__(16) unsigned char cl_dyn[];
-    __shared__ typename L::Shared sh;
-    T *slab = reinterpret_cast<T *>(cl_dyn + C::O_SLAB);
-    int *spos = reinterpret_cast<int *>(cl_dyn + C::O_POS);
-    const int tid = threadIdx.x, rank = blockIdx.x;  // one cluster per launch
+    __shared__ CLeafShared<T, W> sh;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int CL = gridDim.x, rank = blockIdx.x;  // one cluster per launch
     const int c0 = P.c0, w = P.w;
     const int rb = c0 + rank * P.rpc, nr = max(0, min(P.rpc, P.n - rb));
+    const unsigned slab = cl_smem(cl_dyn + C::O_SLAB), ub = cl_smem(cl_dyn + C::O_U), xb = cl_smem(cl_dyn + C::O_X);
+    const unsigned msg = cl_smem(cl_dyn + C::O_MSG), spos = cl_smem(cl_dyn + C::O_POS), out = cl_smem(sh.out);
+    const unsigned cands = cl_smem(&sh.cand[0][0]), bar0 = cl_smem(&sh.bar[0]), failed = cl_smem(&sh.fail);
 
-    // the CTA's rows into their slots, 16 bytes per copy (zeros past column w)
+    // the CTA's rows, 16 bytes per copy (zeros past column w)
     constexpr int CPR = W / VEC;  // copies per row
-    for (int q = tid; q < nr * CPR; q += TPB) {
+    for (int q = tid; q < nr * CPR; q += CL_ALL) {
         const int lr = q / CPR, ch = q % CPR;
-        const int have = min(VEC, max(0, w - ch * VEC)) * (int)sizeof(T);
+        const int have = min(VEC, max(0, w - ch * VEC)) * (int)ES;
         const T *src = P.a + (size_t)(rb + lr) * P.ld + c0 + (have ? ch * VEC : 0);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(cl_smem(slab + lr * PITCH + ch * VEC)),
-                     "l"(src), "r"(have)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(slab + (lr * PITCH + ch * VEC) * ES), "l"(src),
+                     "r"(have)
                      : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     if (tid == 0) {
         sh.fail = *(volatile int *)&P.status[1] != 0;  // an earlier wait of this call gave up: nothing to do
-        for (int b = 0; b < 2; b++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_smem(&sh.bar[b])) : "memory");
+        for (int b = 0; b < 3; b++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * b) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = tid; i < C::ROWB / 4; i += TPB) reinterpret_cast<int *>(sh.none)[i] = 0;
     // the barriers exist before any CTA sends to them
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     __syncthreads();
 
-    typename L::Rows x;
-    const int g0 = tid / S * S, q0 = tid % S;  // row k of this thread's group: k / S * TPB + g0 + k % S
+    // row k of this thread: tid + k CL_TPB of the CTA's (helpers have none)
+    const bool help = tid >= CL_TPB;
+    T r[RT][CL_B];  // its columns of the block from the current one on
+    T ls[RT];       // the multiplier the reference's pivot searches look at
+    int pos[RT];    // its current position (rows of the view); -1: no row
 #pragma unroll
-    for (int k = 0; k < R; k++) {
-        const int lr = k / S * TPB + g0 + k % S;
-#pragma unroll
-        for (int i = 0; i < L::WL; i++) x.r[k][i] = lr < nr ? slab[lr * PITCH + i * S + q0] : T(0);
+    for (int k = 0; k < RT; k++) {
+        pos[k] = !help && tid + k * CL_TPB < nr ? rb + tid + k * CL_TPB : -1;
+        ls[k] = T(0);
     }
-#pragma unroll
-    for (int m = 0; m < L::M; m++) {
-        x.pos[m] = m * TPB + tid < nr ? rb + m * TPB + tid : -1;
-        x.ls[m] = T(0);
-    }
-    __syncwarp();  // a row's slot is written from here on
+    const unsigned slot = slab + tid * PITCH * ES;  // of this thread's first row
+    // this thread's sends of a column's message: piece tid % 8 to CTA tid / 8
+    const int to = tid >> 3, piece = tid & 7;
+    const bool sends = CL > 1 && to < CL && piece < PIECES && rank != P.withhold;
+    const unsigned rmsg = cl_mapa(msg + rank * MSG + piece * 16, sends ? to : 0), rbar = cl_mapa(bar0, sends ? to : 0);
+    // a helper's sends of a pivot row: 16-byte piece lane, to CTAs hw, hw + 4, ...
+    const int hw = warp - CL_NW;
+    const int mode = P.mode, goff = P.goff;
 
-    L::columns(P, sh, cl_dyn, x);
+    bool ok = sh.fail == 0;
+#pragma unroll 1
+    for (int blk = 0; ok && blk < w; blk += CL_B) {
+        const int nbk = min(CL_B, w - blk), rem = w - blk - CL_B;
+        const int rowp = rem > 0 && CL > 1 ? (w - blk + VEC - 1) / VEC : 0;  // 16-byte pieces of a pivot row sent on
+        if (rowp && tid == 0) cl_expect(bar0 + 16, nbk * rowp * 16);
+        if (!help)
+#pragma unroll
+            for (int k = 0; k < RT; k++)
+#pragma unroll
+                for (int j = 0; j < CL_B; j += VEC) {
+                    T v[VEC];
+                    cl_ld16(slot + (k * CL_TPB * PITCH + blk + j) * ES, v);
+#pragma unroll
+                    for (int e = 0; e < VEC; e++) r[k][j + e] = v[e];
+                }
+#pragma unroll 1
+        for (int jb = 0; jb < nbk; jb++) {
+            const int ip = blk + jb, c = c0 + ip, par = ip & 1;
+            if (!help) {
+                const bool use_ls = ip > 0 && ((mode == PIVOT_REF && ((c + goff) & 1)) ||  // lu2tlib.c:1052
+                                               mode == PIVOT_REF_FIRST);
+                // this thread's candidate, the warp's, the CTA's
+                unsigned long long key = 0;
+                int kp = INT_MAX, kr = 0;
+                T kd = T(1);
+#pragma unroll
+                for (int k = 0; k < RT; k++) {
+                    T v = r[k][0];
+                    if (use_ls) v = ls[k];
+                    const int pk = pos[k];
+                    const unsigned long long kk = cl_key(v, pk >= c, pk == c);
+                    const bool take = (kk > key) | ((kk == key) & (pk < kp) & (kk != 0));
+                    key = take ? kk : key;
+                    kp = take ? pk : kp;
+                    kr = take ? k : kr;
+                    kd = take ? r[k][0] : kd;
+                }
+                // the columns after this one scaled, the pivot last: of use to
+                // one lane of the CTA, but made beside the search, not after it
+                T x[CL_B];
+                const T inv = cl_zero(kd) ? T(1) : T(1) / kd;
+#pragma unroll
+                for (int j = 0; j < CL_B; j++) {
+                    x[j] = r[0][(j + 1) % CL_B];
+#pragma unroll
+                    for (int k = 1; k < RT; k++) x[j] = kr == k ? r[k][(j + 1) % CL_B] : x[j];
+                    if (j + 1 < CL_B) x[j] *= inv;
+                }
+                const int wl = cl_winner(key, kp, lane);
+                if (lane == wl) cl_stu(cands + 16 * warp, key, (unsigned)kp);
+                __syncthreads();
+                unsigned long long ck = 0ull, cp = INT_MAX;
+                if (lane < CL_NW) cl_ldu(cands + 16 * lane, ck, cp);
+                if (cl_ldi(failed)) {
+                    ok = false;
+                    break;
+                }
+                if (warp == cl_winner(ck, (int)(unsigned)cp, lane) && lane == wl) {
+                    cl_stu(out, key, (unsigned)kp | (unsigned long long)(unsigned)(tid + kr * CL_TPB) << 32);
+#pragma unroll
+                    for (int j = 0; j < CL_B; j += VEC) {
+                        T v[VEC];
+#pragma unroll
+                        for (int e = 0; e < VEC; e++) v[e] = x[j + e];
+                        cl_st16(out + 16 + j * ES, v);
+                    }
+                }
+            } else {
+                __syncthreads();
+                if (cl_ldi(failed)) {
+                    ok = false;
+                    break;
+                }
+            }
+            __syncthreads();
+            unsigned bst = out;
+            int wc = 0;
+            bool got = true;
+            if (CL > 1) {
+                const unsigned bar = bar0 + 8 * par;
+                if (tid == 0) cl_expect(bar, CL * MSG);
+                if (sends) {
+                    unsigned long long v0, v1;
+                    cl_ldu(out + piece * 16, v0, v1);
+                    cl_send(rmsg + par * CL_MAXC * MSG, v0, v1, rbar + 8 * par);
+                }
+                // every CTA's candidate of this column (after a failed wait what
+                // is read below is nobody's row, and the CTA leaves at its next
+                // barrier: its mbarriers may not be armed again)
+                got = cl_wait(bar, (unsigned)(ip >> 1) & 1u, P.status, P.wait_ns);
+                if (!got) sh.fail = 1;
+                __syncwarp();
+                const unsigned m0 = msg + par * CL_MAXC * MSG;
+                unsigned long long ck = 0ull, cp = INT_MAX;
+                if (lane < CL) cl_ldu(m0 + lane * MSG, ck, cp);
+                wc = cl_winner(ck, (int)(unsigned)cp, lane);
+                bst = m0 + wc * MSG;
+            }
+            const int p = cl_ldi(bst + 8);
+            if (!help) {
+                T u[CL_B];
+#pragma unroll
+                for (int j = 0; j < CL_B; j += VEC) {
+                    T v[VEC];
+                    cl_ld16(bst + 16 + j * ES, v);
+#pragma unroll
+                    for (int e = 0; e < VEC; e++) u[j + e] = v[e];
+                }
+                const bool zero = cl_zero(u[CL_B - 1]);
+#pragma unroll
+                for (int k = 0; k < RT; k++) {
+                    const T l = r[k][0];
+                    const int pk = pos[k];
+                    // rows that are done compute values nobody reads
+                    if (!zero) {
+#pragma unroll
+                        for (int j = 0; j + 1 < CL_B; j++) r[k][j] = cl_fnma(l, u[j], r[k][j + 1]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j + 1 < CL_B; j++) r[k][j] = r[k][j + 1];
+                    }
+                    if ((pk >= c) & (pk != p)) cl_st1(slot + (k * CL_TPB * PITCH + ip) * ES, l);
+                    pos[k] = pk == p ? c : (pk == c ? p : pk);
+                    if (mode == PIVOT_REF || ip == 0) ls[k] = l;
+                }
+            } else {
+                if (rowp) {
+                    // the rest of the pivot row, as it was before the block, and its
+                    // multipliers so far: to all CTAs from its own
+                    if (rank == wc && got && lane < rowp && rank != P.withhold) {
+                        const unsigned row = slab + ((unsigned)cl_ldi(bst + 12) * PITCH + blk) * ES + lane * 16;
+                        unsigned long long v0, v1;
+                        cl_ldu(row, v0, v1);
+#pragma unroll 1
+                        for (int dst = hw; dst < CL; dst += CL_HELP / 32)
+                            cl_send(cl_mapa(xb + (jb * C::XP + blk) * ES + lane * 16, dst), v0, v1,
+                                    cl_mapa(bar0 + 16, dst));
+                    }
+                } else if (hw == 1 && lane == 0) {
+                    sh.row[jb] = CL > 1 ? 0u : slab + (unsigned)cl_ldi(bst + 12) * PITCH * ES;
+                }
+                // row c of the factors, the block's columns from c on
+                if (hw == 0 && lane < CL_B) {
+                    T v;
+                    cl_ld1(bst + 16 + ((lane + CL_B - 1) & (CL_B - 1)) * ES, v);  // the pivot, then the columns after it
+                    if (rank == 0 && lane < nbk - jb) P.a[(size_t)c * P.ld + c + lane] = v;
+                    if (lane == 0) {
+                        sh.d[ip] = v;
+                        sh.piv[ip] = p;
+                    }
+                }
+            }
+        }
+        if (!ok) break;
+        if (!help)
+#pragma unroll
+            for (int k = 0; k < RT; k++)
+                asm volatile("st.shared.s32 [%0], %1;" ::"r"(spos + (tid + k * CL_TPB) * 4), "r"(pos[k]) : "memory");
+        if (rowp && tid < CL_B) sh.row[tid] = xb + tid * C::XP * ES;
+        if (rowp && !cl_wait(bar0 + 16, (unsigned)(blk / CL_B) & 1u, P.status, P.wait_ns)) sh.fail = 1;
+        __syncthreads();
+        if (sh.fail) break;
+        if (rem <= 0) break;  // the last block
+        // the 8 pivot rows right of the block, one column per thread (zeros past
+        // w; whole groups of 8 lanes, whose lanes hold the reciprocals)
+        if (tid < ((rem + 7) & ~7)) {
+            const int col = blk + CL_B + tid;
+            const T dl = sh.d[blk + (lane & (CL_B - 1))], il = cl_zero(dl) ? T(1) : T(1) / dl;
+            const unsigned mates = __activemask();
+            T x[CL_B], lij[CL_B][CL_B];
+#pragma unroll
+            for (int j = 0; j < CL_B; j++) {
+                const unsigned row = (unsigned)cl_ldi(cl_smem(&sh.row[j]));
+                x[j] = T(0);
+                if (tid < rem) cl_ld1(row + col * ES, x[j]);
+#pragma unroll
+                for (int i = 0; i < j; i += VEC) {
+                    T v[VEC];
+                    cl_ld16(row + (blk + i) * ES, v);
+#pragma unroll
+                    for (int e = 0; e < VEC; e++) lij[j][i + e] = v[e];
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < CL_B; j++) {
+                T v = x[j];
+#pragma unroll
+                for (int i = 0; i < j; i++) v = cl_fnma(lij[j][i], x[i], v);
+                v *= __shfl_sync(mates, il, j);
+                if (rank == 0 && tid < rem) P.a[(size_t)(c0 + blk + j) * P.ld + c0 + col] = v;
+                x[j] = cl_zero(__shfl_sync(mates, dl, j)) ? T(0) : v;  // a zero pivot's column subtracts nothing
+                cl_st1(ub + (j * C::UP + tid) * ES, x[j]);
+            }
+        }
+        __syncthreads();
+        if (!help) {
+            if constexpr (sizeof(T) == 8) {
+                const T dz[2] = {sh.d[blk + (lane & 3)], sh.d[blk + (lane & 3) + 4]};
+                cl_update(static_cast<const C *>(nullptr), slab, ub, spos, dz, blk, rem, c0 + blk + CL_B);
+            } else {
+                T dz[CL_B];
+#pragma unroll
+                for (int j = 0; j < CL_B; j++) dz[j] = sh.d[blk + j];
+                cl_update(static_cast<const C *>(nullptr), slab, ub, spos, dz, blk, rem, c0 + blk + CL_B);
+            }
+        }
+        __syncthreads();
+    }
     __syncthreads();
     if (!sh.fail) {
-        // the pivots and their reciprocals, then the multipliers to the rows'
-        // last positions; a pivot row's are scaled by its 1/pivot like the
-        // rest of it, and its columns from its own on are in the matrix already
+        // the pivots, their reciprocals, then the multipliers to the rows' last
+        // positions; a pivot row's are scaled by its 1/pivot like the rest of
+        // it, and its columns from its own on are in the matrix already
         if (tid < w) {
             const T d = sh.d[tid], inv = cl_zero(d) ? T(1) : T(1) / d;
             sh.inv[tid] = inv;
@@ -472,17 +657,14 @@ __global__ void __launch_bounds__(TPB, 1) cluster_leaf_kernel(const CLeafParams<
                 if (cl_zero(d)) atomicMin(&P.status[0], c0 + tid + 1);
             }
         }
-#pragma unroll
-        for (int m = 0; m < L::M; m++)
-            if (m * TPB + tid < nr) spos[m * TPB + tid] = x.pos[m];
         __syncthreads();
-        for (int q = tid; q < nr * CPR; q += TPB) {
+        for (int q = tid; q < nr * CPR; q += CL_ALL) {
             const int lr = q / CPR, ch = q % CPR;
-            const int at = spos[lr], have = min(w, at - c0) - ch * VEC;
+            const int at = cl_ldi(spos + lr * 4), have = min(w, at - c0) - ch * VEC;
             if (have <= 0) continue;
             T *dst = P.a + (size_t)at * P.ld + c0 + ch * VEC;
             T v[VEC];
-            cl_ld16(cl_smem(slab + lr * PITCH + ch * VEC), v);
+            cl_ld16(slab + (lr * PITCH + ch * VEC) * ES, v);
             if (at < c0 + w) {
 #pragma unroll
                 for (int e = 0; e < VEC; e++) v[e] *= sh.inv[at - c0];
@@ -501,59 +683,33 @@ __global__ void __launch_bounds__(TPB, 1) cluster_leaf_kernel(const CLeafParams<
 }
 
 // ---------------------------------------------------------------------------
-// The widest slab one cluster of 16 holds in registers (256 threads of 255), by rows:
+// The widest slab whose rows one cluster of 16 holds, by rows (each CTA
+// 128-170 KB of shared memory):
 //   FP64: 64 columns to 4096 rows, 32 to 8192, 16 to 16384
 //   FP32: 64 columns to 8192 rows, 32 to 16384, 16 to 32768
 // A wider leaf replaces whole levels of the panel recursion (four launches
-// each) by rank-1 steps in registers.  Taller panels go to leaf_kernel.
+// each).  Taller panels go to leaf_kernel.
 template <typename T, int W>
-struct CLeafPick;
-template <>
-struct CLeafPick<double, 64> {
-    static constexpr int S = 4, R = 4, TPB = 256;
-};
-template <>
-struct CLeafPick<double, 32> {
-    static constexpr int S = 4, R = 8, TPB = 256;
-};
-template <>
-struct CLeafPick<double, 16> {
-    static constexpr int S = 2, R = 8, TPB = 256;
-};
-template <>
-struct CLeafPick<float, 64> {
-    static constexpr int S = 4, R = 8, TPB = 256;
-};
-template <>
-struct CLeafPick<float, 32> {
-    static constexpr int S = 4, R = 16, TPB = 256;
-};
-template <>
-struct CLeafPick<float, 16> {
-    static constexpr int S = 2, R = 16, TPB = 256;
-};
-template <typename T, int W>
-using CLeafPickCfg = CLeafCfg<T, W, CLeafPick<T, W>::S, CLeafPick<T, W>::R, CLeafPick<T, W>::TPB>;
+using CLeafPick = CLeafCfg<T, W, 64 / W * (8 / (int)sizeof(T))>;
 
 template <typename T, int W>
 static constexpr int cl_rows()
 {
-    return 16 * CLeafPickCfg<T, W>::ROWS;
+    return CL_MAXC * CLeafPick<T, W>::ROWS;
 }
 
 // shared memory and cluster size limits of one instance; true when a cluster of 16 can be resident
 template <typename T, int W>
 static bool cl_prepare()
 {
-    using K = CLeafPick<T, W>;
-    using C = CLeafPickCfg<T, W>;
-    auto kern = cluster_leaf_kernel<T, W, K::S, K::R, K::TPB>;
+    using C = CLeafPick<T, W>;
+    auto kern = cluster_leaf_kernel<T, W, C::ROWS / CL_TPB>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
         return false;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(16);
-    cfg.blockDim = dim3(K::TPB);
+    cfg.blockDim = dim3(CL_ALL);
     cfg.dynamicSmemBytes = C::SMEM;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -600,8 +756,7 @@ int leaf_width(int rows, size_t tsize, int max_ctas)
 template <typename T, int W>
 static cudaError_t cl_launch_w(CLeafParams<T> P, cudaStream_t st)
 {
-    using K = CLeafPick<T, W>;
-    using C = CLeafPickCfg<T, W>;
+    using C = CLeafPick<T, W>;
     const int rows = P.n - P.c0;
     int cl = 1;
     while (cl < 16 && cl * C::ROWS < rows) cl *= 2;
@@ -609,7 +764,7 @@ static cudaError_t cl_launch_w(CLeafParams<T> P, cudaStream_t st)
     if (P.rpc > C::ROWS) return cudaErrorInvalidConfiguration;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)cl);
-    cfg.blockDim = dim3(K::TPB);
+    cfg.blockDim = dim3(CL_ALL);
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -618,7 +773,7 @@ static cudaError_t cl_launch_w(CLeafParams<T> P, cudaStream_t st)
     cfg.attrs = at;
     cfg.numAttrs = 1;
     count_launch();
-    return cudaLaunchKernelEx(&cfg, cluster_leaf_kernel<T, W, K::S, K::R, K::TPB>, P);
+    return cudaLaunchKernelEx(&cfg, cluster_leaf_kernel<T, W, C::ROWS / CL_TPB>, P);
 }
 
 template <typename T>
