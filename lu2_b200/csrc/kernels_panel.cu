@@ -31,6 +31,10 @@ namespace lu2gpu {
 //           A(k) if p_k = k, else A(j) for the latest j < k with p_j = p_k,
 //           else the original row p_k;
 //   row q >= k1 (some p_j = q) finally holds A(j) for the last such j.
+// The steps that name a row are found through hash lists of the pivots (a
+// linear scan of up to 255 earlier pivots per thread, and jumping rounds that
+// had nothing left to do, took most of the 10.9 us of a launch inside a panel
+// of 8192 rows).
 // Then each CTA gathers the source rows of its column chunks (one 128-byte
 // line per row, 16-byte loads, eight in flight per thread) into shared
 // memory and scatters them to their destinations, scaling the pivot rows.
@@ -39,6 +43,8 @@ namespace lu2gpu {
 // pivots were never written).
 constexpr int SWAP_THREADS = 256;
 constexpr int SWAP_MAX_PIV = 512;
+constexpr int SWAP_HASH = 256;  // lists of pivots by row
+__host__ __device__ constexpr size_t swap_plan_ints(int npiv) { return (size_t)7 * npiv + SWAP_HASH; }
 
 template <typename T, int V>
 struct SwapVec;
@@ -88,11 +94,12 @@ __device__ __forceinline__ void swap_st(T *p, int avail, const T *in)
 // The composed permutation of the exchanges k <-> ipiv[k] - goff, k = k0..k1-1
 // (see above), built by the whole CTA: slot i moves row src[i] to row dst[i];
 // slots 0..npiv-1 are the rows k0..k1-1 (in order), the others the rows >= k1
-// the exchanges name.  P and A: npiv ints each, src and dst: 2 npiv each.
+// the exchanges name.  P, A and nxt: npiv ints each, src and dst: 2 npiv each,
+// head: SWAP_HASH.
 // Returns false (every thread) when the call must do nothing: an earlier wait
 // gave up, or a pivot lies outside [k, nrows) (then ERR_BAD_ARG is recorded).
 __device__ bool swap_plan(const int *__restrict__ ipiv, int goff, int k0, int k1, int nrows, int *P, int *A, int *src,
-                          int *dst, int *p_nslot, int *p_bad, int *status)
+                          int *dst, int *head, int *nxt, int *p_nslot, int *p_bad, int *status)
 {
     const int npiv = k1 - k0, tid = threadIdx.x, nth = blockDim.x;
     int &s_nslot = *p_nslot, &s_bad = *p_bad;
@@ -101,12 +108,14 @@ __device__ bool swap_plan(const int *__restrict__ ipiv, int goff, int k0, int k1
         s_bad = 0;
         s_nslot = npiv;
     }
+    for (int t = tid; t < SWAP_HASH; t += nth) head[t] = -1;
     __syncthreads();
     for (int t = tid; t < npiv; t += nth) {
         const int p = __ldg(ipiv + k0 + t) - goff;
         P[t] = p;
         A[t] = -1;
         if (p < k0 + t || p >= nrows) s_bad = 1;
+        nxt[t] = atomicExch(&head[p & (SWAP_HASH - 1)], t);
     }
     __syncthreads();
     if (s_bad) {
@@ -125,16 +134,19 @@ __device__ bool swap_plan(const int *__restrict__ ipiv, int goff, int k0, int k1
         // pointer jumping, double-buffered through src (free until the slots
         // are written): after r rounds every pointer has advanced 2^r links or
         // reached its root, and a chain has fewer than npiv links
-        int *cur = A, *nxt = src;
+        int *cur = A, *alt = src;
         for (int span = 1; span < npiv; span <<= 1) {
+            bool open = false;
             for (int t = tid; t < npiv; t += nth) {
-                const int v = cur[t];
-                nxt[t] = (v >= 0) ? cur[v] : v;
+                const int v = cur[t], w = (v >= 0) ? cur[v] : v;
+                alt[t] = w;
+                open |= w >= 0;
             }
-            __syncthreads();
+            const bool more = __syncthreads_or(open);
             int *tmp = cur;
-            cur = nxt;
-            nxt = tmp;
+            cur = alt;
+            alt = tmp;
+            if (!more) break;
         }
         if (cur != A) {
             for (int t = tid; t < npiv; t += nth) A[t] = cur[t];
@@ -147,17 +159,19 @@ __device__ bool swap_plan(const int *__restrict__ ipiv, int goff, int k0, int k1
         if (p == k) {
             s = -A[t] - 1;
         } else {
-            int j = t - 1;
-            while (j >= 0 && P[j] != p) j--;
+            // the latest earlier step that names row p, and whether a later one does
+            int j = -1;
+            bool last = true;
+            for (int q = head[p & (SWAP_HASH - 1)]; q >= 0; q = nxt[q]) {
+                if (P[q] != p) continue;
+                if (q < t && q > j) j = q;
+                if (q > t) last = false;
+            }
             s = (j >= 0) ? -A[j] - 1 : p;
-            if (p >= k1) {
-                int q = t + 1;
-                while (q < npiv && P[q] != p) q++;
-                if (q == npiv) {  // the last exchange that names row p
-                    const int e = atomicAdd(&s_nslot, 1);
-                    src[e] = -A[t] - 1;
-                    dst[e] = p;
-                }
+            if (p >= k1 && last) {
+                const int e = atomicAdd(&s_nslot, 1);
+                src[e] = -A[t] - 1;
+                dst[e] = p;
             }
         }
         src[t] = s;
@@ -187,10 +201,11 @@ __global__ void __launch_bounds__(SWAP_THREADS, NS > 0 ? 2 : 1)
     int *A = P + npiv;        // chain pointer (>= 0) or root code -(row)-1
     int *src = A + npiv;      // [2 npiv] source row of each slot
     int *dst = src + 2 * npiv; // [2 npiv] destination row of each slot
+    int *head = dst + 2 * npiv, *nxt = head + SWAP_HASH;  // lists of the pivots by row
     __shared__ int s_nslot, s_bad;
     const int tid = threadIdx.x;
 
-    if (!swap_plan(ipiv, goff, k0, k1, nrows, P, A, src, dst, &s_nslot, &s_bad, status)) return;
+    if (!swap_plan(ipiv, goff, k0, k1, nrows, P, A, src, dst, head, nxt, &s_nslot, &s_bad, status)) return;
     const int nslot = s_nslot;
     const int cq = (tid % TPR) * V, r0 = tid / TPR;
     const int nchunk = (ce - cs + COLS - 1) / COLS;
@@ -264,7 +279,7 @@ static cudaError_t launch_laswp_v(T *a, long ld, int nrows, int k0, int k1, cons
 {
     constexpr int COLS = 128 / (int)sizeof(T);
     const int npiv = k1 - k0;
-    const size_t smem = (NS > 0 ? 0 : (size_t)2 * npiv * COLS * sizeof(T)) + (size_t)6 * npiv * sizeof(int);
+    const size_t smem = (NS > 0 ? 0 : (size_t)2 * npiv * COLS * sizeof(T)) + swap_plan_ints(npiv) * sizeof(int);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(laswp_scale_kernel<T, V, NS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
@@ -331,10 +346,11 @@ __global__ void __launch_bounds__(SWAP_THREADS) solve_inv_kernel(const int *__re
     extern __shared__ __align__(16) int plan_smem[];
     __shared__ int s_nslot, s_bad;
     const int k0 = blockIdx.x * nb, k1 = min(n, k0 + nb), npiv = k1 - k0;
-    int *P = plan_smem, *A = P + npiv, *src = A + npiv, *dst = src + 2 * npiv;
+    int *P = plan_smem, *A = P + npiv, *src = A + npiv, *dst = src + 2 * npiv, *head = dst + 2 * npiv,
+        *nxt = head + SWAP_HASH;
     // (one decision for the CTA; swap_plan without status neither looks nor records)
     if (__syncthreads_or(threadIdx.x == 0 && *(volatile int *)&status[1] != 0)) return;
-    if (!swap_plan(ipiv, 0, k0, k1, n, P, A, src, dst, &s_nslot, &s_bad, nullptr)) {
+    if (!swap_plan(ipiv, 0, k0, k1, n, P, A, src, dst, head, nxt, &s_nslot, &s_bad, nullptr)) {
         if (threadIdx.x == 0) record_error(status, ERR_BAD_ARG, 3);
         return;
     }
@@ -362,7 +378,7 @@ cudaError_t launch_solve_plan(const int *ipiv, int n, int nb, int *inv, int *row
     if (n <= 0 || nb <= 0 || nb > SWAP_MAX_PIV) return cudaErrorInvalidValue;
     const int npan = (n + nb - 1) / nb;
     count_launch(2);
-    solve_inv_kernel<<<npan, SWAP_THREADS, (size_t)6 * nb * sizeof(int), st>>>(ipiv, n, nb, inv, status);
+    solve_inv_kernel<<<npan, SWAP_THREADS, swap_plan_ints(nb) * sizeof(int), st>>>(ipiv, n, nb, inv, status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     solve_rows_kernel<<<(n + SWAP_THREADS - 1) / SWAP_THREADS, SWAP_THREADS, 0, st>>>(inv, n, nb, rows, status);
