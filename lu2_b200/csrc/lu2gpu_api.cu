@@ -881,7 +881,9 @@ extern "C" int lu2gpu_generate(lu2gpu_ctx *c, int n, int nrhs, long seed, int ki
 }
 
 // C = alpha * A * B + beta * C, row-major device matrices (mydgemm's contract
-// on device pointers).  B is transposed into a staging buffer first.
+// on device pointers).  B is transposed into a staging buffer first; A is read
+// in place where the copies by TMA allow it (16-byte aligned, an even stride)
+// and C does not overlap it, else it is copied, too (23 us at m=5000 k=512).
 extern "C" int lu2gpu_dgemm_dev(lu2gpu_ctx *c, int m, int n, int k, double alpha, const double *a, long lda,
                                 const double *b, long ldb, double beta, double *cm, long ldc)
 {
@@ -896,18 +898,24 @@ extern "C" int lu2gpu_dgemm_dev(lu2gpu_ctx *c, int m, int n, int k, double alpha
     const int kk = k > 0 ? k : 1;
     const long ldy = (kk + 1) & ~1L;
     const long ldx = ldy;
-    double *y, *x;
+    const auto first = [](const double *p) { return reinterpret_cast<uintptr_t>(p); };
+    const auto last = [&](const double *p, long ld, int cols) { return first(p) + ((size_t)(m - 1) * ld + cols) * 8; };
+    const bool in_place = k > 0 && !(lda & 1) && !(first(a) & 15) &&
+                          (last(a, lda, k) <= first(cm) || last(cm, ldc, n) <= first(a));
+    double *y, *x = nullptr;
     if ((rc = stage(c, 0, (size_t)n * ldy, &y))) return rc;
-    if ((rc = stage(c, 1, (size_t)m * ldx, &x))) return rc;
+    if (!in_place && (rc = stage(c, 1, (size_t)m * ldx, &x))) return rc;
     if (k == 0) {
         CU_TRY(cudaMemsetAsync(y, 0, (size_t)n * ldy * sizeof(double), c->stream));
         CU_TRY(cudaMemsetAsync(x, 0, (size_t)m * ldx * sizeof(double), c->stream));
     } else {
         K_TRY(launch_transpose(b, ldb, y, ldy, k, n, c->stream));
-        CU_TRY(cudaMemcpy2DAsync(x, ldx * sizeof(double), a, lda * sizeof(double), (size_t)k * sizeof(double), m,
-                                 cudaMemcpyDeviceToDevice, c->stream));
+        if (!in_place)
+            CU_TRY(cudaMemcpy2DAsync(x, ldx * sizeof(double), a, lda * sizeof(double), (size_t)k * sizeof(double), m,
+                                     cudaMemcpyDeviceToDevice, c->stream));
     }
-    K_TRY(launch_dgemm_general(x, ldx, y, ldy, cm, ldc, m, n, kk, alpha, beta, c->d_status, c->stream));
+    K_TRY(launch_dgemm_general(in_place ? a : x, in_place ? lda : ldx, y, ldy, cm, ldc, m, n, kk, alpha, beta,
+                               c->d_status, c->stream));
     return end_status(c, "lu2gpu_dgemm_dev");
 }
 
