@@ -54,7 +54,7 @@ __device__ void batch_solve_smem(double *A, long ld, int n, int nrhs, double *S,
                     p = r;
                 }
             }
-            warp_argmax(v, p);
+            warp_argmax_redux(v, p);
             if (p == INT_MAX) p = k;
             if (p != k)
                 for (int c = lane; c < nc; c += 32) {
@@ -75,10 +75,12 @@ __device__ void batch_solve_smem(double *A, long ld, int n, int nrhs, double *S,
             if (!first_zero) first_zero = k + 1;
             continue;
         }
-        const int w = nc - k - 1, h = n - k - 1;
-        for (int idx = tid; idx < h * w; idx += T) {
-            const int r = k + 1 + idx / w, c = k + 1 + idx % w;
-            S[r * nc + c] -= S[r * nc + k] * S[k * nc + c];
+        // a warp per row (no division of a running index), lanes over its columns;
+        // with the search by integer reductions, 1000 systems of n in [16, 63]:
+        // 213 -> 188 us, [64, 127]: 828 -> 792 us (512 threads, 2 CTAs per SM)
+        for (int r = k + 1 + (tid >> 5); r < n; r += T >> 5) {
+            const double l = S[r * nc + k];
+            for (int c = k + 1 + (tid & 31); c < nc; c += 32) S[r * nc + c] -= l * S[k * nc + c];
         }
         __syncthreads();
     }
@@ -159,8 +161,7 @@ __device__ void batch_solve_blocked(double *A, long ld, int n, int nrhs, int pw,
                         p = r;
                     }
                 }
-                warp_argmax(v, p);
-                if (lane == 0) {
+                if (lane == warp_argmax_redux(v, p)) {
                     s_pv[pw_] = v;
                     s_pi[pw_] = p;
                 }

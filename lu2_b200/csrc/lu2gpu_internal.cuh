@@ -87,6 +87,35 @@ __device__ __forceinline__ void warp_argmax(double &v, int &i)
     }
 }
 
+// The same for candidates v >= 0 (or v < 0: none; never NaN) by three integer
+// reductions on the bits of v (redux.sync, 22 cycles each) instead of five
+// rounds of shuffles of v and i; i in every lane, and the lane that holds it.
+__device__ __forceinline__ int warp_argmax_redux(double v, int &i)
+{
+    const unsigned full = 0xffffffffu;
+    const unsigned hi = v >= 0.0 ? (unsigned)__double2hiint(v) + 1u : 0u, lo = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(full, hi);
+    bool in = hi == mh;
+    const unsigned b = __ballot_sync(full, in);
+    if (b & (b - 1)) {  // a tie in the upper word
+        const unsigned ml = __reduce_max_sync(full, in ? lo : 0u);
+        in = in && lo == ml;
+    }
+    const unsigned mi = __reduce_min_sync(full, in ? (unsigned)i : 0xffffffffu);
+    const unsigned w = __ballot_sync(full, in && (unsigned)i == mi);
+    i = (int)mi;
+    return __ffs(w) - 1;
+}
+__device__ __forceinline__ int warp_argmax_redux(float v, int &i)
+{
+    const unsigned full = 0xffffffffu, k = v >= 0.f ? __float_as_uint(v) + 1u : 0u;
+    const unsigned mk = __reduce_max_sync(full, k);
+    const unsigned mi = __reduce_min_sync(full, k == mk ? (unsigned)i : 0xffffffffu);
+    const unsigned w = __ballot_sync(full, k == mk && (unsigned)i == mi);
+    i = (int)mi;
+    return __ffs(w) - 1;
+}
+
 // ---------------------------------------------------------------------------
 // host-side launchers (all asynchronous on `st`)
 
