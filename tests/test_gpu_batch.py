@@ -242,3 +242,33 @@ def test_objects_left_open_at_exit_are_closed_in_order():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, (r.returncode, r.stderr[-2000:])
+
+
+@pytest.mark.parametrize("pw,ctas", [(16, 1), (16, 2), (24, 1), (64, 1)])
+@pytest.mark.parametrize("nrhs", [1, 2, 8])
+def test_batch_fp32_ir_edge_sizes(ctx, pw, ctas, nrhs):
+    """Orders around the 32-row blocks of the solves, the 8-row tiles of the
+    update, the panel widths and the step from shared to global memory, with
+    the residual recomputed here in extended precision: the refinement stops
+    only when max|r| / (eps n (|A||x| + |b|)) is below 16 (its contract); its
+    own FP64 residual is off by at most (n + 1) eps (|A||x| + |b|), which is
+    1 + 1/n of that unit."""
+    n = np.array([1, 2, 31, 32, 33, 63, 64, 65, 97, 160, 176, 177, 225, 235, 236, 237, 240, 241, 257, 303],
+                 dtype=np.int32)
+    b = L.Batch(ctx, n, np.full(len(n), nrhs, dtype=np.int32))
+    try:
+        b.generate(77)
+        b.snapshot()
+        b.set_mode(L.BATCH_FP32_IR, 10)
+        b.set_config(256, pw, ctas)
+        a0 = [fetch(b, i) for i in range(len(n))]
+        assert (b.solve() == 0).all()
+        assert b.iterations().max() <= 6
+        for i, k in enumerate(int(v) for v in n):
+            a, x = a0[i][:, :k].astype(np.longdouble), fetch(b, i)[:, k:k + nrhs].astype(np.longdouble)
+            rhs = a0[i][:, k:k + nrhs].astype(np.longdouble)
+            r = np.abs(rhs - a @ x).max(axis=0)
+            den = 2.0 ** -53 * k * (np.abs(a).sum(axis=1).max() * np.abs(x).max(axis=0) + np.abs(rhs).max(axis=0))
+            assert (r / den < 17 + 1.01 / k).all(), (k, float((r / den).max()))
+    finally:
+        b.close()
