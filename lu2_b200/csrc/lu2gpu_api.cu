@@ -14,6 +14,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <thread>
 #include <vector>
 
 #include "../../include/lu2gpu.h"
@@ -109,6 +110,9 @@ struct lu2gpu_ctx {
     cudaStream_t h2d_stream = nullptr;
     std::vector<cudaEvent_t> h2d_ev;
     std::vector<cudaEvent_t> blk_ev;  // blocks of the overlapped host-pointer DGEMM
+    // page-locked slots between a pageable host matrix and the device, one event each
+    char *h_slots = nullptr;
+    std::vector<cudaEvent_t> slot_ev;
     // phase timers
     bool timing = false;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev[PH_COUNT];
@@ -297,6 +301,8 @@ extern "C" int lu2gpu_destroy(lu2gpu_ctx *c)
         cudaStreamDestroy(c->h2d_stream);
     }
     for (cudaEvent_t e : c->h2d_ev) cudaEventDestroy(e);
+    for (cudaEvent_t e : c->slot_ev) cudaEventDestroy(e);
+    if (c->h_slots) cudaFreeHost(c->h_slots);
     for (cudaEvent_t e : c->blk_ev) cudaEventDestroy(e);
     free_mixed(c);
     for (int p = 0; p < PH_COUNT; p++)
@@ -1328,6 +1334,11 @@ static int left_looking_panels(int n, int nb)
 // Pageable host matrices at least this large are page-locked by lumcolumn
 // for the call (the copies then overlap the factorization).
 constexpr size_t HOST_REGISTER_MIN_BYTES = (size_t)2 << 30;
+// Smaller pageable ones go through page-locked slots, from this size on (one
+// copy each way -> through the slots, whole calls: n = 700 2.06 -> 1.8 ms,
+// 1000 3.2 -> 2.7, 2048 9.4 -> 5.7, 4096 29.3 -> 14.2, 8192 113 -> 51; n = 512
+// gains less than a tenth, and the slots cost a context some ms once).
+constexpr size_t STAGED_MIN_BYTES = (size_t)4 << 20;
 
 // cudaHostRegister for the duration of one call: take() registers a range;
 // the destructor waits for the context's streams (copies of the range may
@@ -1356,6 +1367,94 @@ struct HostRegistration {
     }
 };
 
+// Copies between a pageable host matrix and the device through page-locked
+// slots of the context (16 of 1 MB): up to 8 threads move the rows between the
+// matrix and their two slots, while the copy engine moves the other slot.  One
+// cudaMemcpy2D of pageable memory stages through one thread: a 2048 x 2049
+// matrix took 3.6 ms to the device and 2.6 ms back (9 and 13 GB/s).
+constexpr size_t SLOT_BYTES = (size_t)1 << 20;
+constexpr int SLOT_THREADS = 8;
+
+// whether the slots serve a matrix of this row length (allocated on first use)
+static bool slots_ready(lu2gpu_ctx *c, size_t row_bytes, int rows)
+{
+    if (row_bytes > SLOT_BYTES || row_bytes * (size_t)rows < STAGED_MIN_BYTES) return false;
+    const size_t need = 2 * SLOT_THREADS;
+    while (c->slot_ev.size() < need) {
+        cudaEvent_t e;
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        c->slot_ev.push_back(e);
+    }
+    if (!c->h_slots && cudaHostAlloc(&c->h_slots, need * SLOT_BYTES, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        c->h_slots = nullptr;
+        return false;
+    }
+    return true;
+}
+
+// rows x row_bytes between host (pitch hp) and device (pitch dp) on the
+// context's stream; back at the caller when the host side is done (the copies
+// to the device may still be in flight, from the slots alone)
+static int staged_copy(lu2gpu_ctx *c, bool to_device, char *host, size_t hp, char *dev, size_t dp, size_t row_bytes,
+                       int rows)
+{
+    const int per = (int)(SLOT_BYTES / row_bytes), chunks = (rows + per - 1) / per;
+    if (!to_device) CU_TRY(cudaStreamSynchronize(c->stream));
+    std::atomic<int> next{0}, failed{cudaSuccess};
+    auto work = [&](int t) {
+        cudaError_t e = cudaSetDevice(c->device);
+        int held[2] = {-1, -1};  // chunk on its way to the host in a slot
+        auto finish = [&](int s) {
+            if (e != cudaSuccess) return;
+            const int slot = 2 * t + s;
+            if ((e = cudaEventSynchronize(c->slot_ev[slot])) != cudaSuccess || held[s] < 0) return;
+            const int r0 = held[s] * per, nr = std::min(per, rows - r0);
+            for (int r = 0; r < nr; ++r)
+                memcpy(host + (size_t)(r0 + r) * hp, c->h_slots + slot * SLOT_BYTES + r * row_bytes, row_bytes);
+            held[s] = -1;
+        };
+        for (int s = 0; e == cudaSuccess && failed.load() == cudaSuccess; s ^= 1) {
+            const int i = next.fetch_add(1);
+            finish(s);  // the slot's copy before, one of an earlier call included
+            if (i >= chunks || e != cudaSuccess) break;
+            const int slot = 2 * t + s, r0 = i * per, nr = std::min(per, rows - r0);
+            char *buf = c->h_slots + slot * SLOT_BYTES, *at = dev + (size_t)r0 * dp;
+            if (to_device) {
+                for (int r = 0; r < nr; ++r) memcpy(buf + r * row_bytes, host + (size_t)(r0 + r) * hp, row_bytes);
+                e = cudaMemcpy2DAsync(at, dp, buf, row_bytes, row_bytes, nr, cudaMemcpyHostToDevice, c->stream);
+            } else {
+                e = cudaMemcpy2DAsync(buf, row_bytes, at, dp, row_bytes, nr, cudaMemcpyDeviceToHost, c->stream);
+                held[s] = i;
+            }
+            if (e == cudaSuccess) e = cudaEventRecord(c->slot_ev[slot], c->stream);
+        }
+        if (!to_device) {
+            finish(0);
+            finish(1);
+        }
+        if (e != cudaSuccess) failed.store(e);
+    };
+    const unsigned cores = std::thread::hardware_concurrency();
+    const int nt = std::max(1, std::min({SLOT_THREADS, (int)cores / 2, chunks}));
+    std::thread pool[SLOT_THREADS];
+    int started = 1;
+    for (; started < nt; ++started) {
+        try {
+            pool[started] = std::thread(work, started);
+        } catch (...) {  // no thread to be had: the others take its rows
+            break;
+        }
+    }
+    work(0);
+    for (int t = 1; t < started; ++t) pool[t].join();
+    CU_TRY((cudaError_t)failed.load());
+    return 0;
+}
+
 static int lumcolumn_host(int n, double *a, double *b, int m, int *pv)
 {
     lu2gpu_ctx *c = default_ctx();
@@ -1382,7 +1481,8 @@ static int lumcolumn_host(int n, double *a, double *b, int m, int *pv)
     // copy stream while the factorization continues; pageable memory would
     // make those copies block the enqueuing thread, so it is copied at the end
     cudaPointerAttributes pa{};
-    bool pinned = cudaPointerGetAttributes(&pa, a) == cudaSuccess && pa.type == cudaMemoryTypeHost;
+    const bool known = cudaPointerGetAttributes(&pa, a) == cudaSuccess;
+    bool pinned = known && pa.type == cudaMemoryTypeHost;
     cudaGetLastError();
     // a large pageable matrix (lu2's main allocates it with malloc or from
     // hugetlbfs, lu2.c:1245-1264) is page-locked for the duration of the call,
@@ -1411,6 +1511,8 @@ static int lumcolumn_host(int n, double *a, double *b, int m, int *pv)
     const int ncol = n + 1;
     const char *ov = getenv("LU2GPU_H2D_OVERLAP");
     const bool overlap = pinned && !(ov && atoi(ov) == 0);
+    const bool staged = !pinned && known && pa.type == cudaMemoryTypeUnregistered &&
+                        slots_ready(c, (size_t)ncol * sizeof(double), n);
     int cw = ncol, p0 = 0, group = 0, waited = 0;
     if (overlap) {
         if (!c->h2d_stream) CU_TRY(cudaStreamCreateWithFlags(&c->h2d_stream, cudaStreamNonBlocking));
@@ -1434,6 +1536,9 @@ static int lumcolumn_host(int n, double *a, double *b, int m, int *pv)
         p0 = lp ? atoi(lp) : left_looking_panels(n, nbw);
         group = (4096 / cw) * cw;
         if (group < cw) group = cw;
+    } else if (staged) {
+        rc = staged_copy(c, true, (char *)a, pitch_h, (char *)d, pitch_d, (size_t)ncol * sizeof(double), n);
+        if (rc) return rc;
     } else {
         CU_TRY(cudaMemcpy2DAsync(d, pitch_d, a, pitch_h, (size_t)ncol * sizeof(double), n, cudaMemcpyHostToDevice,
                                  c->stream));
@@ -1467,6 +1572,9 @@ static int lumcolumn_host(int n, double *a, double *b, int m, int *pv)
     if (pinned) {
         CU_TRY(cudaEventRecord(c->copy_ev, c->copy_stream));
         CU_TRY(cudaStreamWaitEvent(c->stream, c->copy_ev, 0));
+    } else if (staged) {
+        rc = staged_copy(c, false, (char *)a, pitch_h, (char *)d, pitch_d, (size_t)ncol * sizeof(double), n);
+        if (rc) return rc;
     } else {
         CU_TRY(cudaMemcpy2DAsync(a, pitch_h, d, pitch_d, (size_t)(n + 1) * sizeof(double), n, cudaMemcpyDeviceToHost,
                                  c->stream));
