@@ -366,8 +366,19 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParam
                 }
             };
             if constexpr (!EXACT) {
-                c[0] = c[1] = c[2] = c[3] = 0.0;
-                products();
+                // four chains of 16 products: one chain of 64 left a backward
+                // error of x up to half larger (n = 2048, 16 systems, geometric
+                // mean: 6.1e-16 against 4.6e-16)
+                double s[4][4];
+#pragma unroll
+                for (int b = 0; b < 4; b++) s[b][0] = s[b][1] = s[b][2] = s[b][3] = 0.0;
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const double2 x = *reinterpret_cast<const double2 *>(xg + 8 * j + 2 * t);
+                    ts_mma(s[j & 3], v[4 * j], v[4 * j + 2], v[4 * j + 1], v[4 * j + 3], -x.x, -x.y);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e++) c[e] = (s[0][e] + s[1][e]) + (s[2][e] + s[3][e]);
                 double *q0 = part_sum + tr0 * NR + 2 * t, *q1 = q0 + 8 * NR;
                 if (half == 1) {
                     q0[0] = c[0];
