@@ -398,12 +398,12 @@ constexpr int TRSM_TLD = TRSM_BK + 1;
 
 // T: the unit lower triangle (strict lower part used), row stride ldt; X: the
 // K x ncols block (row stride ldx) solved in place; bt (optional) receives
-// X^T * bt_scale converted to BT (double, float or bf16), negated when bt_neg
-// (the FP64 trailing update reads -U12^T and adds).
-template <typename E, typename BT>
-__global__ void __launch_bounds__(256) trsm_unit_lower_kernel(const E *T, long ldt, E *Xg, long ldx, int K, int ncols,
-                                                              BT *bt, const float *bt_scale, int bt_neg)
+// -X^T (the FP64 trailing update reads -U12^T and adds).  FP64, for what
+// trsm_dmma_kernel does not take.
+__global__ void __launch_bounds__(256)
+    trsm_unit_lower_kernel(const double *T, long ldt, double *Xg, long ldx, int K, int ncols, double *bt)
 {
+    using E = double;
     extern __shared__ __align__(16) unsigned char trsm_smem[];
     E *X = reinterpret_cast<E *>(trsm_smem);  // K x TRSM_LDS, then Ts: K x TRSM_TLD
     E *Ts = X + (size_t)K * TRSM_LDS;
@@ -469,15 +469,203 @@ __global__ void __launch_bounds__(256) trsm_unit_lower_kernel(const E *T, long l
     for (int r = rg; r < K; r += 8)
         if (jok) Xg[(size_t)r * ldx + j] = X[r * TRSM_LDS + col];
     if (!bt) return;
-    const float sc = bt_scale ? *bt_scale : 1.0f;
     const int jbase = blockIdx.x * TRSM_TW;
     for (int idx = threadIdx.x; idx < TRSM_TW * K; idx += 256) {
         const int cc = idx / K, r = idx - cc * K;
-        if (jbase + cc < ncols) {
-            const E v = X[r * TRSM_LDS + cc];
-            bt[(size_t)(jbase + cc) * K + r] = bt_scale ? (BT)(float)(v * (E)sc) : (BT)(bt_neg ? -v : v);
+        if (jbase + cc < ncols) bt[(size_t)(jbase + cc) * K + r] = -X[r * TRSM_LDS + cc];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The same solve in FP32, the same operations in the same order per element,
+// for the precision forms: 32 CPL columns per CTA, all K rows of them in
+// shared memory, T's 16-column blocks copied one step ahead (cp.async).  The
+// first CPL warps substitute through a diagonal block, a column per lane; then
+// the products with the rows below run in register tiles of 8 x 4 CPL.
+// What bounds it is the shared-memory pipe and the chain of 16-row steps.  A
+// column per lane (the FP64 kernel above) reads a value of T for each product,
+// and a broadcast feeds two values a cycle to an SM whose cores take four.
+// K = 256, in the FP64 kernel's manner -> here: 4704 columns 51 -> 25 us, 9472
+// 67 -> 35, 12032 89 -> 58; K = 512, 4700 columns 115 -> 64 (with a lane one
+// column, T four values at a time and prefetched: 31, 41, 55, 86).
+constexpr int T32_BK = 16;
+constexpr int T32_TP = T32_BK + 4;  // pitch of a staged T block: rows 16-byte aligned
+
+template <int CPL>
+struct T32Cfg {
+    static constexpr int COLS = 32 * CPL;
+    static constexpr int P = COLS + 4;  // pitch of X
+    static constexpr size_t smem(int K)
+    {
+        return ((size_t)K * P + 2 * (size_t)(K < T32_BK ? T32_BK : K) * T32_TP) * sizeof(float);
+    }
+};
+
+// n (1 or 4) floats to shared memory, `have` of them from src, the rest zeros
+__device__ __forceinline__ void t32_copy(float *dst, const float *src, int n, int have)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if (n == 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(4 * have) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(4 * have) : "memory");
+}
+
+template <int CPL>
+__global__ void __launch_bounds__(256, 2)
+    trsm_f32_kernel(const float *__restrict__ T, long ldt, float *Xg, long ldx, int K, int ncols, float *bt, int tvec,
+                    int xvec)
+{
+    using C = T32Cfg<CPL>;
+    constexpr int P = C::P, COLS = C::COLS, CT = COLS / 8;  // CT: columns of a thread in the products
+    extern __shared__ __align__(16) unsigned char t32_smem[];
+    float *X = reinterpret_cast<float *>(t32_smem);  // [K][P]
+    float *Ts = X + (size_t)K * P;                   // [2][max(K, 16)][T32_TP]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int j0 = blockIdx.x * COLS, nc = min(COLS, ncols - j0), tsz = max(K, T32_BK) * T32_TP;
+
+    // columns lb .. lb + 15 of T from row lb on (zeros past K)
+    auto stage = [&](int lb) {
+        float *dst = Ts + ((lb / T32_BK) & 1) * tsz;
+        const int bk = min(T32_BK, K - lb), per = tvec ? 4 : 1, sh = tvec ? 2 : 4;  // copies per row: 1 << sh
+        for (int q = tid; q < (K - lb) << sh; q += 256) {
+            const int r = q >> sh, c = (q & ((1 << sh) - 1)) * per, have = max(0, min(per, bk - c));
+            t32_copy(dst + r * T32_TP + c, T + (size_t)(lb + r) * ldt + lb + (have ? c : 0), per, have);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    {
+        const int per = xvec ? 4 : 1, pr = COLS / per;
+        for (int q = tid; q < K * pr; q += 256) {
+            const int r = q / pr, c = q % pr * per, have = max(0, min(per, nc - c));
+            t32_copy(X + r * P + c, Xg + (size_t)r * ldx + j0 + (have ? c : 0), per, have);
         }
     }
+    stage(0);
+    for (int lb = 0; lb < K; lb += T32_BK) {
+        const int bk = min(T32_BK, K - lb);
+        const float *Tc = Ts + ((lb / T32_BK) & 1) * tsz;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // the block has arrived, and the step before is done
+        if (lb + T32_BK < K) stage(lb + T32_BK);
+        if (warp < CPL) {
+            float *x = X + lb * P + 32 * warp + lane;
+            float xd[T32_BK];
+#pragma unroll
+            for (int l = 0; l < T32_BK; l++) xd[l] = l < bk ? x[l * P] : 0.f;
+#pragma unroll
+            for (int l0 = 0; l0 < T32_BK; l0 += 4) {
+                // columns l0 .. l0 + 3: rows of the block read four values at
+                // a time (rows past K hold anything; nothing reads their x)
+#pragma unroll
+                for (int r = l0 + 1; r < T32_BK; r++) {
+                    const float4 t = *reinterpret_cast<const float4 *>(Tc + r * T32_TP + l0);
+                    xd[r] -= t.x * xd[l0];
+                    if (r > l0 + 1) xd[r] -= t.y * xd[l0 + 1];
+                    if (r > l0 + 2) xd[r] -= t.z * xd[l0 + 2];
+                    if (r > l0 + 3) xd[r] -= t.w * xd[l0 + 3];
+                }
+            }
+#pragma unroll
+            for (int l = 0; l < T32_BK; l++)
+                if (l < bk) x[l * P] = xd[l];
+        }
+        if (lb + T32_BK >= K) break;  // (bk == 16 from here on)
+        __syncthreads();
+        // rows below, 32 per warp at a time: a thread 8 of them (every fourth,
+        // so that a quarter-warp's rows of T lie on distinct banks) by CT columns
+        const int rg = lane >> 3, cg = 4 * (lane & 7);
+        for (int rw = lb + T32_BK + 32 * warp; rw < K; rw += 256) {
+            float s[8][CT];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int e = 0; e < CT; e++) s[i][e] = 0.f;
+            const float *tr = Tc + (rw + rg - lb) * T32_TP;
+            const int last = K - 1 - rw - rg;  // rows past K read one of the matrix
+#pragma unroll
+            for (int l = 0; l < T32_BK; l += 4) {
+                float4 t[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    t[i] = *reinterpret_cast<const float4 *>(tr + (4 * i <= last ? 4 * i : 0) * T32_TP + l);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float xv[CT];
+#pragma unroll
+                    for (int e = 0; e < CT; e += 4)
+                        *reinterpret_cast<float4 *>(xv + e) =
+                            *reinterpret_cast<const float4 *>(X + (lb + l + q) * P + 8 * e + cg);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const float tv = q == 0 ? t[i].x : q == 1 ? t[i].y : q == 2 ? t[i].z : t[i].w;
+#pragma unroll
+                        for (int e = 0; e < CT; e++) s[i][e] += tv * xv[e];
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (4 * i <= last) {
+#pragma unroll
+                    for (int e = 0; e < CT; e += 4) {
+                        float4 *x = reinterpret_cast<float4 *>(X + (rw + rg + 4 * i) * P + 8 * e + cg);
+                        float4 v = *x;
+                        v.x -= s[i][e];
+                        v.y -= s[i][e + 1];
+                        v.z -= s[i][e + 2];
+                        v.w -= s[i][e + 3];
+                        *x = v;
+                    }
+                }
+        }
+    }
+    __syncthreads();
+    if (xvec && nc == COLS) {
+        for (int q = tid; q < K * (COLS / 4); q += 256) {
+            const int r = q / (COLS / 4), c = q % (COLS / 4) * 4;
+            *reinterpret_cast<float4 *>(Xg + (size_t)r * ldx + j0 + c) = *reinterpret_cast<const float4 *>(X + r * P + c);
+        }
+    } else {
+        for (int q = tid; q < K * COLS; q += 256) {
+            const int r = q / COLS, c = q % COLS;
+            if (c < nc) Xg[(size_t)r * ldx + j0 + c] = X[r * P + c];
+        }
+    }
+    if (!bt) return;
+    // X^T, 8 rows of a column per thread where they are whole sectors
+    if ((K & 7) == 0 && (reinterpret_cast<uintptr_t>(bt) & 15) == 0) {
+        for (int q = tid; q < (K >> 3) * COLS; q += 256) {
+            const int c = q % COLS, r = q / COLS * 8;
+            if (c < nc) {
+                float4 *o = reinterpret_cast<float4 *>(bt + (size_t)(j0 + c) * K + r);
+                const float *x = X + r * P + c;
+                o[0] = make_float4(x[0], x[P], x[2 * P], x[3 * P]);
+                o[1] = make_float4(x[4 * P], x[5 * P], x[6 * P], x[7 * P]);
+            }
+        }
+    } else {
+        for (int q = tid; q < K * COLS; q += 256) {
+            const int c = q / K, r = q - c * K;
+            if (c < nc) bt[(size_t)(j0 + c) * K + r] = X[r * P + c];
+        }
+    }
+}
+
+template <int CPL>
+static cudaError_t launch_trsm_f32_t(const float *t, long ldt, float *x, long ldx, int K, int ncols, float *bt,
+                                     cudaStream_t st)
+{
+    const size_t smem = T32Cfg<CPL>::smem(K);
+    if (smem > 227 * 1024) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(trsm_f32_kernel<CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
+    const int tvec = (reinterpret_cast<uintptr_t>(t) & 15) == 0 && (ldt & 3) == 0;
+    const int xvec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (ldx & 3) == 0;
+    count_launch();
+    trsm_f32_kernel<CPL><<<(ncols + T32Cfg<CPL>::COLS - 1) / T32Cfg<CPL>::COLS, 256, smem, st>>>(t, ldt, x, ldx, K,
+                                                                                              ncols, bt, tvec, xvec);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -671,21 +859,19 @@ static cudaError_t launch_trsm_dmma(const double *t, long ldt, double *x, long l
     return cudaGetLastError();
 }
 
-template <typename E, typename BT>
-static cudaError_t launch_trsm_t(const E *t, long ldt, E *x, long ldx, int K, int ncols, BT *bt, const float *bt_scale, int bt_neg,
-                                 cudaStream_t st)
+static cudaError_t launch_trsm_cores(const double *t, long ldt, double *x, long ldx, int K, int ncols, double *bt,
+                                     cudaStream_t st)
 {
-    if (ncols <= 0 || K <= 0) return cudaSuccess;
-    const size_t smem = (size_t)K * (TRSM_LDS + TRSM_TLD) * sizeof(E);
+    const size_t smem = (size_t)K * (TRSM_LDS + TRSM_TLD) * sizeof(double);
     if (smem > 210 * 1024) return cudaErrorInvalidValue;
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(trsm_unit_lower_kernel<E, BT>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024);
+        cudaError_t e =
+            cudaFuncSetAttribute(trsm_unit_lower_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024);
         if (e != cudaSuccess) return e;
     }
     const int blocks = (ncols + TRSM_TW - 1) / TRSM_TW;
     count_launch();
-    trsm_unit_lower_kernel<E, BT><<<blocks, 256, smem, st>>>(t, ldt, x, ldx, K, ncols, bt, bt_scale, bt_neg);
+    trsm_unit_lower_kernel<<<blocks, 256, smem, st>>>(t, ldt, x, ldx, K, ncols, bt);
     return cudaGetLastError();
 }
 
@@ -699,7 +885,7 @@ cudaError_t launch_trsm_unit_lower_tx(const double *t, long ldt, double *x, long
         use_dmma = (e && e[0] == '0') ? 0 : 1;
     }
     if (use_dmma && trsm_dmma_ok(t, ldt, x, ldx, K, ncols, bt)) return launch_trsm_dmma(t, ldt, x, ldx, K, ncols, bt, st);
-    return launch_trsm_t<double, double>(t, ldt, x, ldx, K, ncols, bt, nullptr, 1, st);
+    return launch_trsm_cores(t, ldt, x, ldx, K, ncols, bt, st);
 }
 
 cudaError_t launch_trsm_unit_lower(double *a, long ld, int r0, int K, int cs, int ce, double *bt, cudaStream_t st)
@@ -707,16 +893,14 @@ cudaError_t launch_trsm_unit_lower(double *a, long ld, int r0, int K, int cs, in
     return launch_trsm_unit_lower_tx(a + (size_t)r0 * ld + r0, ld, a + (size_t)r0 * ld + cs, ld, K, ce - cs, bt, st);
 }
 
+// 32 columns per CTA while all CTAs are resident at once (two per SM: 25 us at
+// K = 256 with one, 35 with two), else 64 (one round of 58 us to 18944 columns).
 cudaError_t launch_trsm_unit_lower_f32(const float *t, long ldt, float *x, long ldx, int K, int ncols, float *bt,
                                        cudaStream_t st)
 {
-    return launch_trsm_t<float, float>(t, ldt, x, ldx, K, ncols, bt, nullptr, 0, st);
-}
-
-cudaError_t launch_trsm_unit_lower_f32_bf16(const float *t, long ldt, float *x, long ldx, int K, int ncols, void *bt,
-                                            const float *bt_scale, cudaStream_t st)
-{
-    return launch_trsm_t<float, __nv_bfloat16>(t, ldt, x, ldx, K, ncols, (__nv_bfloat16 *)bt, bt_scale, 0, st);
+    if (ncols <= 0 || K <= 0) return cudaSuccess;
+    return ncols > 2 * 148 * 32 ? launch_trsm_f32_t<2>(t, ldt, x, ldx, K, ncols, bt, st)
+                                : launch_trsm_f32_t<1>(t, ldt, x, ldx, K, ncols, bt, st);
 }
 
 }  // namespace lu2gpu

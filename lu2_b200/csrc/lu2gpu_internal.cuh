@@ -179,12 +179,9 @@ cudaError_t launch_trsm_unit_lower(double *a, long ld, int r0, int K, int cs, in
 // (row stride ldx) given separately; bt may be null.
 cudaError_t launch_trsm_unit_lower_tx(const double *t, long ldt, double *x, long ldx, int K, int ncols, double *bt,
                                       cudaStream_t st);
-// FP32 versions for the precision form; the _bf16 one writes the transposed
-// block row as BF16 multiplied by *bt_scale (a device scalar).
+// FP32 version for the precision forms; bt receives X^T.
 cudaError_t launch_trsm_unit_lower_f32(const float *t, long ldt, float *x, long ldx, int K, int ncols, float *bt,
                                        cudaStream_t st);
-cudaError_t launch_trsm_unit_lower_f32_bf16(const float *t, long ldt, float *x, long ldx, int K, int ncols, void *bt,
-                                            const float *bt_scale, cudaStream_t st);
 
 // C[m][n] += sum_k A[m][k] * Bt[n][k] with Bt = -U12^T (as the block solve
 // writes it), i.e. the trailing update C - L21 U12.  A is the
