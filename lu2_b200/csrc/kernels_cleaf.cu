@@ -380,7 +380,10 @@ __device__ __forceinline__ void cl_update(const CLeafCfg<float, W, RT> *, unsign
     }
 }
 
-template <typename T, int W, int RT>
+// REF: one of the reference's pivot rules, whose searches look at multipliers
+// (64 columns by plain partial pivoting without them in the chain: 200 rows
+// 56 -> 52 us, 4096 rows 79.5 -> 77)
+template <typename T, int W, int RT, bool REF>
 __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafParams<T> P)
 {
     using C = CLeafCfg<T, W, RT>;
@@ -458,8 +461,8 @@ __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafPara
         for (int jb = 0; jb < nbk; jb++) {
             const int ip = blk + jb, c = c0 + ip, par = ip & 1;
             if (!help) {
-                const bool use_ls = ip > 0 && ((mode == PIVOT_REF && ((c + goff) & 1)) ||  // lu2tlib.c:1052
-                                               mode == PIVOT_REF_FIRST);
+                const bool use_ls = REF && ip > 0 &&
+                                    (mode == PIVOT_REF_FIRST || ((c + goff) & 1));  // lu2tlib.c:1052
                 // this thread's candidate, the warp's, the CTA's
                 unsigned long long key = 0;
                 int kp = INT_MAX, kr = 0;
@@ -562,7 +565,7 @@ __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafPara
                     }
                     if ((pk >= c) & (pk != p)) cl_st1(slot + (k * CL_TPB * PITCH + ip) * ES, l);
                     pos[k] = pk == p ? c : (pk == c ? p : pk);
-                    if (mode == PIVOT_REF || ip == 0) ls[k] = l;
+                    if (REF && (mode == PIVOT_REF || ip == 0)) ls[k] = l;
                 }
             } else {
                 if (rowp) {
@@ -703,11 +706,11 @@ static constexpr int cl_rows()
 }
 
 // shared memory and cluster size limits of one instance; true when a cluster of 16 can be resident
-template <typename T, int W>
-static bool cl_prepare()
+template <typename T, int W, bool REF>
+static bool cl_prepare_1()
 {
     using C = CLeafPick<T, W>;
-    auto kern = cluster_leaf_kernel<T, W, C::ROWS / CL_TPB>;
+    auto kern = cluster_leaf_kernel<T, W, C::ROWS / CL_TPB, REF>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
         return false;
@@ -722,6 +725,12 @@ static bool cl_prepare()
     cfg.numAttrs = 1;
     int clusters = 0;
     return cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters >= 1;
+}
+
+template <typename T, int W>
+static bool cl_prepare()
+{
+    return cl_prepare_1<T, W, false>() && cl_prepare_1<T, W, true>();
 }
 
 // whether the current device takes the cluster leaf (looked up once per device)
@@ -777,7 +786,8 @@ static cudaError_t cl_launch_w(CLeafParams<T> P, cudaStream_t st)
     cfg.attrs = at;
     cfg.numAttrs = 1;
     count_launch();
-    return cudaLaunchKernelEx(&cfg, cluster_leaf_kernel<T, W, C::ROWS / CL_TPB>, P);
+    return P.mode == PIVOT_PARTIAL ? cudaLaunchKernelEx(&cfg, cluster_leaf_kernel<T, W, C::ROWS / CL_TPB, false>, P)
+                                   : cudaLaunchKernelEx(&cfg, cluster_leaf_kernel<T, W, C::ROWS / CL_TPB, true>, P);
 }
 
 template <typename T>
