@@ -284,7 +284,7 @@ __device__ __forceinline__ void cl_update(const CLeafCfg<double, W, RT> *, unsig
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int pg = (g >> 1) + ((g & 1) << 2);
     const unsigned r0 = slab + (warp * 32 * RT + pg) * C::PITCH * 8;
-    constexpr int MT = RT > 2 ? 4 : 2 * RT;  // tiles at a time
+    constexpr int MT = RT > 1 && RT % 2 ? 2 : RT > 2 ? 4 : 2 * RT;  // tiles at a time
 #pragma unroll 1
     for (int pass = 0; pass < 2 * RT / MT; pass++) {
         const unsigned rp = r0 + pass * MT * 16 * C::PITCH * 8;
@@ -340,15 +340,17 @@ __device__ __forceinline__ void cl_update(const CLeafCfg<float, W, RT> *, unsign
                                           const float (&dz)[8], int blk, int rem, int c1)
 {
     using C = CLeafCfg<float, W, RT>;
-    // each thread its own rows, two at a time
+    // each thread its own rows, two or three at a time
+    constexpr int RU = RT % 2 ? 3 : 2;
+    static_assert(RT % RU == 0, "whole groups of rows");
     const int tid = threadIdx.x;
 #pragma unroll
-    for (int k = 0; k < RT; k += 2) {
-        float l[2][CL_B];
-        unsigned row[2];
-        bool live[2];
+    for (int k = 0; k < RT; k += RU) {
+        float l[RU][CL_B];
+        unsigned row[RU];
+        bool live[RU];
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
+        for (int h = 0; h < RU; h++) {
             const int lr = tid + (k + h) * CL_TPB;
             row[h] = slab + (lr * C::PITCH + blk) * 4;
             live[h] = cl_ldi(spos + lr * 4) >= c1;
@@ -362,20 +364,21 @@ __device__ __forceinline__ void cl_update(const CLeafCfg<float, W, RT> *, unsign
         }
 #pragma unroll 1
         for (int n0 = 0; n0 < rem; n0 += 4) {
-            float c[2][4];
-            cl_ld16(row[0] + (CL_B + n0) * 4, c[0]);
-            cl_ld16(row[1] + (CL_B + n0) * 4, c[1]);
+            float c[RU][4];
+#pragma unroll
+            for (int h = 0; h < RU; h++) cl_ld16(row[h] + (CL_B + n0) * 4, c[h]);
 #pragma unroll
             for (int j = 0; j < CL_B; j++) {
                 float u[4];
                 cl_ld16(ub + (j * C::UP + n0) * 4, u);
 #pragma unroll
-                for (int h = 0; h < 2; h++)
+                for (int h = 0; h < RU; h++)
 #pragma unroll
                     for (int e = 0; e < 4; e++) c[h][e] = cl_fnma(l[h][j], u[e], c[h][e]);
             }
-            if (live[0]) cl_st16(row[0] + (CL_B + n0) * 4, c[0]);
-            if (live[1]) cl_st16(row[1] + (CL_B + n0) * 4, c[1]);
+#pragma unroll
+            for (int h = 0; h < RU; h++)
+                if (live[h]) cl_st16(row[h] + (CL_B + n0) * 4, c[h]);
         }
     }
 }
@@ -691,25 +694,28 @@ __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafPara
 
 // ---------------------------------------------------------------------------
 // The widest slab whose rows one cluster of 16 holds, by rows (each CTA
-// 128-170 KB of shared memory):
-//   FP64: 64 columns to 4096 rows, 32 to 8192, 16 to 16384
-//   FP32: 64 columns to 8192 rows, 32 to 16384, 16 to 32768
+// 128-170 KB of shared memory, the tall instances 210-226 KB):
+//   FP64: 64 columns to 4096 rows, 32 to 8192, tall 12288, 16 to 16384, tall 20480
+//   FP32: 64 columns to 8192 rows, tall 12288, 32 to 16384, tall 24576, 16 to 32768
 // A wider leaf replaces whole levels of the panel recursion (four launches
-// each).  Taller panels go to leaf_kernel.
-template <typename T, int W>
-using CLeafPick = CLeafCfg<T, W, 64 / W * (8 / (int)sizeof(T))>;
+// each).  The tall instances fill the SM's shared memory (FP32, 12288 rows: 64
+// columns 90 us against twice 51 and those launches; FP64: 32 columns 57
+// against twice 34; 16 columns of about 20000 rows beside an update 33 us,
+// over the whole grid 151).  Taller panels go to leaf_kernel.
+template <typename T, int W, bool TALL>
+using CLeafPick = CLeafCfg<T, W, sizeof(T) == 8 ? (TALL ? 64 / W + 1 : 64 / W) : (TALL ? 192 / W : 128 / W)>;
 
-template <typename T, int W>
+template <typename T, int W, bool TALL>
 static constexpr int cl_rows()
 {
-    return CL_MAXC * CLeafPick<T, W>::ROWS;
+    return CL_MAXC * CLeafPick<T, W, TALL>::ROWS;
 }
 
 // shared memory and cluster size limits of one instance; true when a cluster of 16 can be resident
-template <typename T, int W, bool REF>
+template <typename T, int W, bool TALL, bool REF>
 static bool cl_prepare_1()
 {
-    using C = CLeafPick<T, W>;
+    using C = CLeafPick<T, W, TALL>;
     auto kern = cluster_leaf_kernel<T, W, C::ROWS / CL_TPB, REF>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
@@ -727,10 +733,10 @@ static bool cl_prepare_1()
     return cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters >= 1;
 }
 
-template <typename T, int W>
+template <typename T, int W, bool TALL = false>
 static bool cl_prepare()
 {
-    return cl_prepare_1<T, W, false>() && cl_prepare_1<T, W, true>();
+    return cl_prepare_1<T, W, TALL, false>() && cl_prepare_1<T, W, TALL, true>();
 }
 
 // whether the current device takes the cluster leaf (looked up once per device)
@@ -742,7 +748,9 @@ static bool cl_device_ok()
     signed char k = known[dev].load();
     if (k == 0) {
         k = cl_prepare<double, 64>() && cl_prepare<double, 32>() && cl_prepare<double, 16>() &&
-                    cl_prepare<float, 64>() && cl_prepare<float, 32>() && cl_prepare<float, 16>()
+                    cl_prepare<float, 64>() && cl_prepare<float, 32>() && cl_prepare<float, 16>() &&
+                    cl_prepare<double, 32, true>() && cl_prepare<double, 16, true>() &&
+                    cl_prepare<float, 64, true>() && cl_prepare<float, 32, true>()
                 ? 1
                 : -1;
         cudaGetLastError();
@@ -751,25 +759,34 @@ static bool cl_device_ok()
     return k > 0;
 }
 
+// columns the leaf takes for `rows` rows, in the tall instance or not; 0: not this leaf
 template <typename T>
-static int cl_width(int rows, int max_ctas)
+static int cl_width(int rows, int max_ctas, bool &tall)
 {
+    tall = false;
     if (rows <= 0 || max_ctas < 16 || !cl_device_ok()) return 0;
-    if (rows <= cl_rows<T, 64>()) return 64;
-    if (rows <= cl_rows<T, 32>()) return 32;
-    return rows <= cl_rows<T, 16>() ? 16 : 0;
+    if (rows <= cl_rows<T, 64, false>()) return 64;
+    tall = sizeof(T) == 4 && rows <= cl_rows<float, 64, true>();
+    if (tall) return 64;
+    if (rows <= cl_rows<T, 32, false>()) return 32;
+    tall = rows <= cl_rows<T, 32, true>();
+    if (tall) return 32;
+    if (rows <= cl_rows<T, 16, false>()) return 16;
+    tall = sizeof(T) == 8 && rows <= cl_rows<double, 16, true>();
+    return tall ? 16 : 0;
 }
 
 int leaf_width(int rows, size_t tsize, int max_ctas)
 {
-    const int k = tsize == sizeof(double) ? cl_width<double>(rows, max_ctas) : cl_width<float>(rows, max_ctas);
+    bool tall;
+    const int k = tsize == sizeof(double) ? cl_width<double>(rows, max_ctas, tall) : cl_width<float>(rows, max_ctas, tall);
     return k > 16 ? k : 16;
 }
 
-template <typename T, int W>
+template <typename T, int W, bool TALL = false>
 static cudaError_t cl_launch_w(CLeafParams<T> P, cudaStream_t st)
 {
-    using C = CLeafPick<T, W>;
+    using C = CLeafPick<T, W, TALL>;
     const int rows = P.n - P.c0;
     int cl = 1;
     while (cl < 16 && cl * C::ROWS < rows) cl *= 2;
@@ -796,14 +813,21 @@ static cudaError_t launch_leaf_cluster_t(T *a, long ld, int n, int c0, int w, in
                                          bool *used)
 {
     *used = false;
-    const int width = cl_width<T>(n - c0, max_ctas);
+    bool tall;
+    const int width = cl_width<T>(n - c0, max_ctas, tall);
     constexpr int VEC = 16 / (int)sizeof(T);
     // 16-byte copies of row segments
     if (w <= 0 || w > width || (reinterpret_cast<uintptr_t>(a) & 15) || ld % VEC || c0 % VEC) return cudaSuccess;
     *used = true;
     const CLeafParams<T> P{a, ld, n, c0, w, 0, mode, goff, ipiv, dinv, status, buf.wait_ns, buf.withhold};
-    if (w <= 16) return cl_launch_w<T, 16>(P, st);
-    return w <= 32 ? cl_launch_w<T, 32>(P, st) : cl_launch_w<T, 64>(P, st);
+    // a narrower slab has more rows in its base instance than a wider tall one
+    if (w <= 16 && n - c0 <= cl_rows<T, 16, false>()) return cl_launch_w<T, 16>(P, st);
+    if (w <= 32 && n - c0 <= cl_rows<T, 32, false>()) return cl_launch_w<T, 32>(P, st);
+    if (!tall) return cl_launch_w<T, 64>(P, st);
+    if constexpr (sizeof(T) == 8)
+        return width == 16 ? cl_launch_w<T, 16, true>(P, st) : cl_launch_w<T, 32, true>(P, st);
+    else
+        return width == 32 ? cl_launch_w<T, 32, true>(P, st) : cl_launch_w<T, 64, true>(P, st);
 }
 
 cudaError_t launch_leaf_cluster(double *a, long ld, int n, int c0, int w, int mode, int goff, int *ipiv, double *dinv,

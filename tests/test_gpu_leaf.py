@@ -113,3 +113,29 @@ def test_fp32_leaf_with_several_rows_per_thread(ctx, n):
     assert ctx.lusolve(a, n, ld, 256) == 0
     x64 = a[:, n]
     assert float((x - x64).abs().max() / x64.abs().max()) <= 2 * 16 * n * U * 4
+
+
+@pytest.mark.parametrize("n,m", [(8193, 32), (8200, 17), (12288, 32), (12289, 16), (16385, 16), (20480, 16),
+                                 (20481, 16)])
+@pytest.mark.parametrize("mode", [L.PIVOT_PARTIAL, L.PIVOT_REF])
+def test_tall_leaf_edges(n, m, mode):
+    """The instances with more rows per CTA, at both ends of their rows."""
+    a = np.random.default_rng(n + m).uniform(-0.5, 0.5, (n, m))
+    if mode == L.PIVOT_REF:  # its odd columns' pivots need not be large: keep the growth small
+        a[np.arange(m), np.arange(m)] += m
+    old = L.set_pivot_mode(mode)
+    try:
+        f, pv = factor(a, m)
+    finally:
+        L.set_pivot_mode(old)
+    check(a, f, pv)
+    if mode == L.PIVOT_PARTIAL:
+        assert np.all(np.abs(f[m:]) <= np.abs(f[np.arange(m), np.arange(m)]))
+    else:
+        assert np.all(pv[::2] >= np.arange(0, m, 2)) and pv[0] == np.argmax(np.abs(a[:, 0]))
+
+
+@pytest.mark.parametrize("n", [8193, 12288, 12289, 24576])
+def test_fp32_tall_leaf_edges(ctx, n):
+    """The FP32 tall instances' first and last row counts, as above."""
+    test_fp32_leaf_with_several_rows_per_thread(ctx, n)
