@@ -10,49 +10,109 @@ namespace lu2gpu {
 
 // ---------------------------------------------------------------------------
 // C -= A Bt^T in FP32 on the CUDA cores (exact FP32 arithmetic for the panel,
-// which the precision form keeps in FP32).  64 x 64 tiles, 256 threads of 4 x 4.
+// which the precision form keeps in FP32).  64 x 64 tiles, 256 threads of 4 x 4,
+// each sum over k from zero and subtracted once.
+// These updates have K = 64 or 128 and a few hundred tiles, so that the trips
+// to memory bound them: C is read before the products, the next 32 columns of
+// A and Bt beside them (16-byte loads where VEC: rows 16-byte aligned, K a
+// multiple of 4), two buffers in shared memory.  The operands lie there k-major
+// with row r of column k at r ^ 4 (k / 4), which puts a warp's transposing
+// stores on distinct banks and keeps four rows together.
+// One slab at a time, read value by value and C last -> this: M = 4000, N = K =
+// 64 9.6 -> 5.0 us, N = K = 128 15.4 -> 8.5; M = 12000, 128 22.4 -> 16.7.
 constexpr int SG_T = 64, SG_K = 32;
 
+template <bool VEC>
 __global__ void __launch_bounds__(256) sgemm_update_kernel(const float *__restrict__ a, long lda,
                                                            const float *__restrict__ bt, float *c, long ldc, int M,
                                                            int N, int K)
 {
-    __shared__ float As[SG_K][SG_T + 4];
-    __shared__ float Bs[SG_K][SG_T + 4];
-    const int m0 = blockIdx.x * SG_T, n0 = blockIdx.y * SG_T;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += SG_K) {
-        for (int idx = threadIdx.x; idx < SG_T * SG_K; idx += 256) {
-            const int r = idx / SG_K, k = idx - r * SG_K;
-            const int gk = k0 + k;
-            As[k][r] = (m0 + r < M && gk < K) ? a[(size_t)(m0 + r) * lda + gk] : 0.f;
-            Bs[k][r] = (n0 + r < N && gk < K) ? bt[(size_t)(n0 + r) * K + gk] : 0.f;
+    __shared__ __align__(16) float As[2][SG_K * SG_T], Bs[2][SG_K * SG_T];
+    const int m0 = blockIdx.x * SG_T, n0 = blockIdx.y * SG_T, tid = threadIdx.x;
+    const int tx = tid & 15, ty = tid >> 4;
+    // this thread's C: rows m0 + 4 ty + i, columns n0 + 4 tx + j
+    const bool cvec = VEC && n0 + SG_T <= N && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0;
+    float *cp = c + (size_t)(m0 + 4 * ty) * ldc + n0 + 4 * tx;
+    float old[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        if (cvec && m0 + 4 * ty + i < M) {
+            const float4 v = *reinterpret_cast<const float4 *>(cp + (size_t)i * ldc);
+            old[i][0] = v.x;
+            old[i][1] = v.y;
+            old[i][2] = v.z;
+            old[i][3] = v.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                old[i][j] = m0 + 4 * ty + i < M && n0 + 4 * tx + j < N ? cp[(size_t)i * ldc + j] : 0.f;
         }
-        __syncthreads();
+    }
+    // this thread's part of a slab: rows tid / 8 and + 32, columns 4 (tid % 8) ..
+    const int sr = tid >> 3, sk = 4 * (tid & 7);
+    float4 ra[2], rb[2];
+    auto fetch = [&](const float *p, long ld, int row0, int rows, int k0, float4 (&v)[2]) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int r = row0 + sr + 32 * h, k = k0 + sk;
+            const float *q = p + (size_t)r * ld + k;
+            if (VEC)
+                v[h] = r < rows && k < K ? *reinterpret_cast<const float4 *>(q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            else
+                v[h] = make_float4(r < rows && k < K ? q[0] : 0.f, r < rows && k + 1 < K ? q[1] : 0.f,
+                                   r < rows && k + 2 < K ? q[2] : 0.f, r < rows && k + 3 < K ? q[3] : 0.f);
+        }
+    };
+    auto load = [&](int k0) {
+        fetch(a, lda, m0, M, k0, ra);
+        fetch(bt, K, n0, N, k0, rb);
+    };
+    auto store = [&](int buf) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int r = (sr + 32 * h) ^ sk;
+            float *pa = As[buf] + sk * SG_T + r, *pb = Bs[buf] + sk * SG_T + r;
+            pa[0] = ra[h].x;
+            pa[SG_T] = ra[h].y;
+            pa[2 * SG_T] = ra[h].z;
+            pa[3 * SG_T] = ra[h].w;
+            pb[0] = rb[h].x;
+            pb[SG_T] = rb[h].y;
+            pb[2 * SG_T] = rb[h].z;
+            pb[3 * SG_T] = rb[h].w;
+        }
+    };
+    float acc[4][4] = {};
+    load(0);
+    store(0);
+    __syncthreads();
+    for (int k0 = 0, buf = 0; k0 < K; k0 += SG_K, buf ^= 1) {
+        const bool more = k0 + SG_K < K;
+        if (more) load(k0 + SG_K);
 #pragma unroll 8
         for (int k = 0; k < SG_K; k++) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                av[i] = As[k][ty * 4 + i];
-                bv[i] = Bs[k][tx * 4 + i];
-            }
+            const int sw = k & ~3;
+            const float4 av = *reinterpret_cast<const float4 *>(As[buf] + k * SG_T + ((4 * ty) ^ sw));
+            const float4 bv = *reinterpret_cast<const float4 *>(Bs[buf] + k * SG_T + ((4 * tx) ^ sw));
+            const float x[4] = {av.x, av.y, av.z, av.w}, y[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
         }
+        if (more) store(buf ^ 1);
         __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= M) continue;
+        if (m0 + 4 * ty + i >= M) continue;
+        if (cvec) {
+            *reinterpret_cast<float4 *>(cp + (size_t)i * ldc) = make_float4(
+                old[i][0] - acc[i][0], old[i][1] - acc[i][1], old[i][2] - acc[i][2], old[i][3] - acc[i][3]);
+        } else {
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
-            if (n < N) c[(size_t)m * ldc + n] -= acc[i][j];
+            for (int j = 0; j < 4; j++)
+                if (n0 + 4 * tx + j < N) cp[(size_t)i * ldc + j] = old[i][j] - acc[i][j];
         }
     }
 }
@@ -64,7 +124,12 @@ cudaError_t launch_sgemm_update(const float *a, long lda, const float *bt, float
     dim3 grid((M + SG_T - 1) / SG_T, (N + SG_T - 1) / SG_T);
     if (grid.y > 65535) return cudaErrorInvalidConfiguration;
     count_launch();
-    sgemm_update_kernel<<<grid, 256, 0, st>>>(a, lda, bt, c, ldc, M, N, K);
+    const bool vec = (reinterpret_cast<uintptr_t>(a) & 15) == 0 && (lda & 3) == 0 &&
+                     (reinterpret_cast<uintptr_t>(bt) & 15) == 0 && (K & 3) == 0;
+    if (vec)
+        sgemm_update_kernel<true><<<grid, 256, 0, st>>>(a, lda, bt, c, ldc, M, N, K);
+    else
+        sgemm_update_kernel<false><<<grid, 256, 0, st>>>(a, lda, bt, c, ldc, M, N, K);
     return cudaGetLastError();
 }
 
