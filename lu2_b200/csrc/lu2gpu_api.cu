@@ -2193,8 +2193,7 @@ static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, in
     {
         PhaseTimer t(c, PH_DGEMM);
         CU_TRY(cudaMemsetAsync(m->amax(), 0, 2 * sizeof(unsigned), c->stream));
-        K_TRY(launch_absmax(L, v.ld, M, K, m->amax(), c->stream));
-        K_TRY(launch_absmax(X, v.ld, K, N, m->amax() + 1, c->stream));
+        K_TRY(launch_absmax2(L, v.ld, M, K, X, v.ld, K, N, m->amax(), c->stream));
         K_TRY(launch_panel_scales(m->amax(), m->scales(), c->stream));
         K_TRY(launch_f32_to_bf16(L, v.ld, m->l16, K, M, K, m->scales(), c->stream));
         K_TRY(launch_f32_transpose_bf16(X, v.ld, K, N, m->u16, m->scales() + 1, c->stream));

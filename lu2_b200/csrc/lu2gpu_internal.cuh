@@ -253,8 +253,9 @@ cudaError_t launch_sgemm_update(const float *a, long lda, const float *bt, float
                                 cudaStream_t st);
 // per-panel power-of-two scales for the BF16 operands: scales[0] = 1/sL,
 // scales[1] = 1/sU, scales[2] = sL*sU with sX = 2^ceil(log2(max|X|)) of the
-// rows x cols block X (called once per block; amax[] accumulates maxima)
-cudaError_t launch_absmax(const float *x, long ld, int rows, int cols, unsigned *amax_bits, cudaStream_t st);
+// rows x cols block X (amax[0], amax[1] accumulate the two blocks' maxima)
+cudaError_t launch_absmax2(const float *x0, long ld0, int rows0, int cols0, const float *x1, long ld1, int rows1,
+                           int cols1, unsigned *amax_bits, cudaStream_t st);
 cudaError_t launch_panel_scales(const unsigned *amax_bits, float *scales, cudaStream_t st);
 // y = FP32(x) for an n x cols FP64 block and back
 cudaError_t launch_f64_to_f32(const double *x, long ldx, float *y, long ldy, int rows, int cols, cudaStream_t st);
