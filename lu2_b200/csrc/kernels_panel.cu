@@ -11,6 +11,8 @@
 
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "lu2gpu_internal.cuh"
 
 namespace lu2gpu {
@@ -185,11 +187,14 @@ __device__ bool swap_plan(const int *__restrict__ ipiv, int goff, int k0, int k1
 // (all NS loads in flight at once, one barrier per chunk, no staging in
 // shared memory; used while the slots fit, nslot <= NS * rows per pass);
 // NS = 0: the chunk is staged in shared memory.
+// blockIdx.y: the job; jobs share no column, so their CTAs are independent.
 template <typename T, int V, int NS>
 __global__ void __launch_bounds__(SWAP_THREADS, NS > 0 ? 2 : 1)
-    laswp_scale_kernel(T *a, long ld, int nrows, int k0, int k1, const int *__restrict__ ipiv, int goff,
-                       const T *__restrict__ dinv, int cs, int ce, int scale, int *status)
+    laswp_scale_kernel(T *a, long ld, int nrows, const __grid_constant__ SwapJobs jobs, const int *__restrict__ ipiv,
+                       int goff, const T *__restrict__ dinv, int scale, int *status)
 {
+    const SwapJob &job = jobs.j[blockIdx.y];
+    const int k0 = job.k0, k1 = job.k1, cs = job.cs, ce = job.ce;
     constexpr int COLS = 128 / (int)sizeof(T);  // one 128-byte line of a row per chunk
     constexpr int TPR = COLS / V;               // threads per row segment
     constexpr int RPP = SWAP_THREADS / TPR;     // rows per pass
@@ -274,11 +279,15 @@ __global__ void __launch_bounds__(SWAP_THREADS, NS > 0 ? 2 : 1)
 }
 
 template <typename T, int V, int NS>
-static cudaError_t launch_laswp_v(T *a, long ld, int nrows, int k0, int k1, const int *ipiv, int goff, const T *dinv,
-                                  int cs, int ce, bool scale, int *status, cudaStream_t st)
+static cudaError_t launch_laswp_v(T *a, long ld, int nrows, const SwapJobs &jobs, const int *ipiv, int goff,
+                                  const T *dinv, bool scale, int *status, cudaStream_t st)
 {
     constexpr int COLS = 128 / (int)sizeof(T);
-    const int npiv = k1 - k0;
+    int npiv = 0, width = 0;
+    for (int q = 0; q < jobs.n; q++) {
+        npiv = std::max(npiv, jobs.j[q].k1 - jobs.j[q].k0);
+        width = std::max(width, jobs.j[q].ce - jobs.j[q].cs);
+    }
     const size_t smem = (NS > 0 ? 0 : (size_t)2 * npiv * COLS * sizeof(T)) + swap_plan_ints(npiv) * sizeof(int);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(laswp_scale_kernel<T, V, NS>,
@@ -290,37 +299,66 @@ static cudaError_t launch_laswp_v(T *a, long ld, int nrows, int k0, int k1, cons
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int per_sm = NS > 0 ? 2 : (int)((220 * 1024) / (smem + 1024));
     per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
-    int blocks = (ce - cs + COLS - 1) / COLS;
+    int blocks = (width + COLS - 1) / COLS;
     if (blocks > per_sm * sms) blocks = per_sm * sms;
     count_launch();
-    laswp_scale_kernel<T, V, NS><<<blocks, SWAP_THREADS, smem, st>>>(a, ld, nrows, k0, k1, ipiv, goff, dinv, cs,
-                                                                      ce, scale ? 1 : 0, status);
+    laswp_scale_kernel<T, V, NS><<<dim3((unsigned)blocks, (unsigned)jobs.n), SWAP_THREADS, smem, st>>>(
+        a, ld, nrows, jobs, ipiv, goff, dinv, scale ? 1 : 0, status);
     return cudaGetLastError();
 }
 
 // registers while 2 npiv slots fit NS passes of SWAP_THREADS / (COLS / V) rows
 template <typename T, int V>
-static cudaError_t launch_laswp_pick(T *a, long ld, int nrows, int k0, int k1, const int *ipiv, int goff,
-                                     const T *dinv, int cs, int ce, bool scale, int *status, cudaStream_t st)
+static cudaError_t launch_laswp_pick(T *a, long ld, int nrows, const SwapJobs &jobs, const int *ipiv, int goff,
+                                     const T *dinv, bool scale, int *status, cudaStream_t st)
 {
     constexpr int RPP = SWAP_THREADS / ((128 / (int)sizeof(T)) / V);
     constexpr int NSR = (V > 1) ? 16 : 0;  // 16 passes: 512 slots (npiv <= 256) at 16-byte accesses
-    if (NSR > 0 && 2 * (k1 - k0) <= NSR * RPP)
-        return launch_laswp_v<T, V, NSR>(a, ld, nrows, k0, k1, ipiv, goff, dinv, cs, ce, scale, status, st);
-    return launch_laswp_v<T, V, 0>(a, ld, nrows, k0, k1, ipiv, goff, dinv, cs, ce, scale, status, st);
+    bool few = NSR > 0;
+    for (int q = 0; q < jobs.n; q++) few = few && 2 * (jobs.j[q].k1 - jobs.j[q].k0) <= NSR * RPP;
+    if (few) return launch_laswp_v<T, V, NSR>(a, ld, nrows, jobs, ipiv, goff, dinv, scale, status, st);
+    return launch_laswp_v<T, V, 0>(a, ld, nrows, jobs, ipiv, goff, dinv, scale, status, st);
+}
+
+template <typename T>
+static cudaError_t launch_laswp_t(T *a, long ld, int nrows, const SwapJobs &all, const int *ipiv, int goff,
+                                  const T *dinv, bool scale, int *status, cudaStream_t st)
+{
+    constexpr int VW = 16 / (int)sizeof(T);
+    SwapJobs jobs;
+    // 16-byte accesses when every row segment starts on a 16-byte boundary
+    bool vec = (reinterpret_cast<uintptr_t>(a) & 15) == 0 && ld % VW == 0;
+    for (int q = 0; q < all.n; q++) {
+        const SwapJob &j = all.j[q];
+        if (j.ce <= j.cs || j.k1 <= j.k0) continue;
+        if (j.k1 - j.k0 > SWAP_MAX_PIV || j.k0 < 0 || j.k1 > nrows) return cudaErrorInvalidValue;
+        vec = vec && j.cs % VW == 0;
+        jobs.j[jobs.n++] = j;
+    }
+    if (jobs.n == 0) return cudaSuccess;
+    if (vec) return launch_laswp_pick<T, VW>(a, ld, nrows, jobs, ipiv, goff, dinv, scale, status, st);
+    return launch_laswp_pick<T, 1>(a, ld, nrows, jobs, ipiv, goff, dinv, scale, status, st);
 }
 
 template <typename T>
 static cudaError_t launch_laswp_scale_t(T *a, long ld, int nrows, int k0, int k1, const int *ipiv, int goff,
                                         const T *dinv, int cs, int ce, bool scale, int *status, cudaStream_t st)
 {
-    if (ce <= cs || k1 <= k0) return cudaSuccess;
-    if (k1 - k0 > SWAP_MAX_PIV || k0 < 0 || k1 > nrows) return cudaErrorInvalidValue;
-    constexpr int VW = 16 / (int)sizeof(T);
-    // 16-byte accesses when every row segment starts on a 16-byte boundary
-    if ((reinterpret_cast<uintptr_t>(a) & 15) == 0 && ld % VW == 0 && cs % VW == 0)
-        return launch_laswp_pick<T, VW>(a, ld, nrows, k0, k1, ipiv, goff, dinv, cs, ce, scale, status, st);
-    return launch_laswp_pick<T, 1>(a, ld, nrows, k0, k1, ipiv, goff, dinv, cs, ce, scale, status, st);
+    SwapJobs one;
+    one.add(k0, k1, cs, ce);
+    return launch_laswp_t(a, ld, nrows, one, ipiv, goff, dinv, scale, status, st);
+}
+
+cudaError_t launch_laswp_jobs(double *a, long ld, int nrows, const SwapJobs &jobs, const int *ipiv, int goff,
+                              const double *dinv, int *status, cudaStream_t st)
+{
+    return launch_laswp_t(a, ld, nrows, jobs, ipiv, goff, dinv, true, status, st);
+}
+
+cudaError_t launch_laswp_jobs(float *a, long ld, int nrows, const SwapJobs &jobs, const int *ipiv, int goff,
+                              const float *dinv, int *status, cudaStream_t st)
+{
+    return launch_laswp_t(a, ld, nrows, jobs, ipiv, goff, dinv, true, status, st);
 }
 
 cudaError_t launch_laswp_scale(double *a, long ld, int nrows, int k0, int k1, const int *ipiv, int goff,

@@ -464,17 +464,28 @@ struct View {
         }                                                                                             \
     } while (0)
 
-// Pivots of view columns k0..k1 applied to columns cs..ce, then U rows solved
-// and the rows below updated (lu2.c:524-581 / lu2tlib.c:1068-1093).
-static int right_part(lu2gpu_ctx *c, const View &v, int k0, int k1, int cs, int ce, bool top)
+static int swap_rows_now(lu2gpu_ctx *c, const View &v, const SwapJobs &jobs)
 {
-    if (ce <= cs) return 0;
+    if (jobs.n)
+        K_TRY(launch_laswp_jobs(v.a, v.ld, v.n, jobs, c->d_ipiv + v.goff, v.goff, c->d_dinv + v.goff, c->d_status,
+                                c->stream));
+    return 0;
+}
+
+// Pivots of view columns k0..k1 applied to columns cs..ce (and the exchanges
+// `left` that panels before have put off), then U rows solved and the rows below
+// updated (lu2.c:524-581 / lu2tlib.c:1068-1093).
+static int right_part(lu2gpu_ctx *c, const View &v, int k0, int k1, int cs, int ce, bool top,
+                      SwapJobs left = SwapJobs())
+{
+    if (ce <= cs) return swap_rows_now(c, v, left);
     int *ipiv = c->d_ipiv + v.goff;
     double *dinv = c->d_dinv + v.goff;
     const int K = k1 - k0;
     {
         PhaseTimer t(c, top ? PH_SWAP : PH_PANEL);
-        K_TRY(launch_laswp_scale(v.a, v.ld, v.n, k0, k1, ipiv, v.goff, dinv, cs, ce, true, c->d_status, c->stream));
+        left.add(k0, k1, cs, ce);
+        K_TRY(launch_laswp_jobs(v.a, v.ld, v.n, left, ipiv, v.goff, dinv, c->d_status, c->stream));
     }
     // inner right parts of a panel (K x (ce - cs) <= nb^2 / 4) use their own
     // buffer, so that a panel factored beside a running update (which reads
@@ -501,12 +512,13 @@ static int right_part(lu2gpu_ctx *c, const View &v, int k0, int k1, int cs, int 
 // cs + w1: `hook` runs between the update of columns cs..cs+w1-1 and that of
 // the rest (the lookahead factors the next panel there)
 template <typename Hook>
-static int right_part_split(lu2gpu_ctx *c, const View &v, int k0, int k1, int cs, int ce, int w1, Hook hook)
+static int right_part_split(lu2gpu_ctx *c, const View &v, int k0, int k1, int cs, int ce, int w1, SwapJobs left,
+                            Hook hook)
 {
-    if (ce <= cs) return hook();
+    if (ce > cs) left.add(k0, k1, cs, ce);
+    const int rs = swap_rows_now(c, v, left);
+    if (rs || ce <= cs) return rs ? rs : hook();
     const int K = k1 - k0;
-    K_TRY(launch_laswp_scale(v.a, v.ld, v.n, k0, k1, c->d_ipiv + v.goff, v.goff, c->d_dinv + v.goff, cs, ce, true,
-                             c->d_status, c->stream));
     K_TRY(launch_trsm_unit_lower(v.a, v.ld, k0, K, cs, ce, c->d_bt, c->stream));
     if (k1 >= v.n) return hook();
     if (w1 > ce - cs) w1 = ce - cs;
@@ -522,7 +534,13 @@ static int right_part_split(lu2gpu_ctx *c, const View &v, int k0, int k1, int cs
 
 // Recursive panel (lu2.c:1088-1120): columns c0..c0+m-1, rows c0..n-1.  The
 // split keeps every left width a multiple of 16 (the GEMM's K step).
-static int panel(lu2gpu_ctx *c, const View &v, int c0, int m, int mode)
+// A right half's exchanges on the left half's columns are put off to the next
+// launch of exchanges that comes anyway (`left`): nothing reads those columns
+// before the update that follows it, and no two of them share a column.  Each
+// was a launch of its own on the chain of panels, 5-7 us, three in a panel of
+// 256 with 64-column leaves (n = 3333: 6.00 -> 5.87 ms without them, n = 8192:
+// 24.8 -> 24.15).
+static int panel_rec(lu2gpu_ctx *c, const View &v, int c0, int m, int mode, SwapJobs &left)
 {
     if (m <= leaf_width(v.n - c0, sizeof(double), c->leaf_ctas)) {
         PhaseTimer t(c, PH_LEAF);
@@ -532,16 +550,25 @@ static int panel(lu2gpu_ctx *c, const View &v, int c0, int m, int mode)
     }
     int h = ((m / 2) + 15) & ~15;
     if (h >= m) h = m - 16;
-    int rc = panel(c, v, c0, h, mode);
+    SwapJobs inner;
+    int rc = panel_rec(c, v, c0, h, mode, inner);
     if (rc) return rc;
-    rc = right_part(c, v, c0, c0 + h, c0 + h, c0 + m, false);
+    rc = right_part(c, v, c0, c0 + h, c0 + h, c0 + m, false, inner);
     if (rc) return rc;
-    rc = panel(c, v, c0 + h, m - h, mode);
+    rc = panel_rec(c, v, c0 + h, m - h, mode, left);
+    if (rc) return rc;
+    left.add(c0 + h, c0 + m, c0, c0 + h);
+    return 0;
+}
+
+// The panel with every exchange in place.
+static int panel(lu2gpu_ctx *c, const View &v, int c0, int m, int mode)
+{
+    SwapJobs left;
+    const int rc = panel_rec(c, v, c0, m, mode, left);
     if (rc) return rc;
     PhaseTimer t(c, PH_PANEL);
-    K_TRY(launch_laswp_scale(v.a, v.ld, v.n, c0 + h, c0 + m, c->d_ipiv + v.goff, v.goff, c->d_dinv + v.goff, c0,
-                             c0 + h, true, c->d_status, c->stream));
-    return 0;
+    return swap_rows_now(c, v, left);
 }
 
 static int ensure_work(lu2gpu_ctx *c, int n, int ncols, int nb)
@@ -645,7 +672,8 @@ static int factor_lookahead(lu2gpu_ctx *c, const View &v, int i0, int nb, int mo
     }
     const cudaStream_t main_st = c->stream;
     const int all_ctas = c->leaf_ctas;
-    int rc = panel(c, v, i0, std::min(nb, n - i0), mode);  // the first panel, on the main stream
+    SwapJobs left;  // the factored panel's exchanges on its own columns, done with its right part's
+    int rc = panel_rec(c, v, i0, std::min(nb, n - i0), mode, left);  // the first panel, on the main stream
     for (int i = i0; rc == 0 && i < n; i += nb) {
         const int w = std::min(nb, n - i), i1 = i + w, w1 = std::min(nb, n - i1);
         if (i > i0 && cudaStreamWaitEvent(main_st, c->ev_panel, 0) != cudaSuccess) {
@@ -659,14 +687,15 @@ static int factor_lookahead(lu2gpu_ctx *c, const View &v, int i0, int nb, int mo
             CU_TRY(cudaStreamWaitEvent(c->side, c->ev_cols, 0));
             c->stream = c->side;
             c->leaf_ctas = std::min(all_ctas, std::max(LOOKAHEAD_LEAF_CTAS, leaf_min_ctas(n - i1, sizeof(double))));
-            const int r = panel(c, v, i1, w1, mode);
+            left = SwapJobs();
+            const int r = panel_rec(c, v, i1, w1, mode, left);
             c->stream = main_st;
             c->leaf_ctas = all_ctas;
             if (r) return r;
             CU_TRY(cudaEventRecord(c->ev_panel, c->side));
             return 0;
         };
-        rc = right_part_split(c, v, i, i1, i1, v.ncols, w1, next_panel);
+        rc = right_part_split(c, v, i, i1, i1, v.ncols, w1, left, next_panel);
         if (!rc) rc = after_step(i, w);
     }
     c->stream = main_st;
@@ -2113,19 +2142,29 @@ struct View32 {
 // (the lookahead hook), then the rest; update kernels capped at max_ctas CTAs.
 template <typename Hook>
 static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, int cs, int ce, int w1, int max_ctas,
-                              Hook after_first);
+                              SwapJobs left, Hook after_first);
 
-static int right_part32(lu2gpu_ctx *c, const View32 &v, int k0, int k1, int cs, int ce, bool top)
+static int swap_rows_now32(lu2gpu_ctx *c, const View32 &v, const SwapJobs &jobs)
 {
-    if (ce <= cs) return 0;
-    if (top) return right_part32_split(c, v, k0, k1, cs, ce, 0, 0, []() { return 0; });
+    if (jobs.n)
+        K_TRY(launch_laswp_jobs(v.a, v.ld, v.n, jobs, c->d_ipiv + v.goff, v.goff, c->mx->dinv + v.goff, c->d_status,
+                                c->stream));
+    return 0;
+}
+
+static int right_part32(lu2gpu_ctx *c, const View32 &v, int k0, int k1, int cs, int ce, bool top,
+                        SwapJobs left = SwapJobs())
+{
+    if (ce <= cs) return swap_rows_now32(c, v, left);
+    if (top) return right_part32_split(c, v, k0, k1, cs, ce, 0, 0, left, []() { return 0; });
     MixedWork *m = c->mx;
     int *ipiv = c->d_ipiv + v.goff;
     float *dinv = m->dinv + v.goff;
     const int K = k1 - k0;
     {
         PhaseTimer t(c, top ? PH_SWAP : PH_PANEL);
-        K_TRY(launch_laswp_scale(v.a, v.ld, v.n, k0, k1, ipiv, v.goff, dinv, cs, ce, true, c->d_status, c->stream));
+        left.add(k0, k1, cs, ce);
+        K_TRY(launch_laswp_jobs(v.a, v.ld, v.n, left, ipiv, v.goff, dinv, c->d_status, c->stream));
     }
     const float *T = v.a + (size_t)k0 * v.ld + k0;
     float *X = v.a + (size_t)k0 * v.ld + cs;
@@ -2141,18 +2180,21 @@ static int right_part32(lu2gpu_ctx *c, const View32 &v, int k0, int k1, int cs, 
 
 template <typename Hook>
 static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, int cs, int ce, int w1, int max_ctas,
-                              Hook after_first)
+                              SwapJobs left, Hook after_first)
 {
-    if (ce <= cs) return after_first();
+    if (ce <= cs) {
+        const int rs = swap_rows_now32(c, v, left);
+        return rs ? rs : after_first();
+    }
     MixedWork *m = c->mx;
-    int *ipiv = c->d_ipiv + v.goff;
-    float *dinv = m->dinv + v.goff;
     const int K = k1 - k0, M = v.n - k1, N = ce - cs;
     // the second launch starts at a quantization tile boundary of U12^T
     if (w1 <= 0 || w1 >= N || (w1 % 128)) w1 = N;
     {
         PhaseTimer t(c, PH_SWAP);
-        K_TRY(launch_laswp_scale(v.a, v.ld, v.n, k0, k1, ipiv, v.goff, dinv, cs, ce, true, c->d_status, c->stream));
+        left.add(k0, k1, cs, ce);
+        const int rs = swap_rows_now32(c, v, left);
+        if (rs) return rs;
     }
     const float *T = v.a + (size_t)k0 * v.ld + k0;
     float *X = v.a + (size_t)k0 * v.ld + cs;
@@ -2210,7 +2252,7 @@ static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, in
     return 0;
 }
 
-static int panel32(lu2gpu_ctx *c, const View32 &v, int c0, int m, int mode)
+static int panel32_rec(lu2gpu_ctx *c, const View32 &v, int c0, int m, int mode, SwapJobs &left)
 {
     if (m <= leaf_width(v.n - c0, sizeof(float), c->leaf_ctas)) {
         PhaseTimer t(c, PH_LEAF);
@@ -2220,14 +2262,22 @@ static int panel32(lu2gpu_ctx *c, const View32 &v, int c0, int m, int mode)
     }
     int h = ((m / 2) + 15) & ~15;
     if (h >= m) h = m - 16;
-    int rc = panel32(c, v, c0, h, mode);
+    SwapJobs inner;
+    int rc = panel32_rec(c, v, c0, h, mode, inner);
     if (rc) return rc;
-    if ((rc = right_part32(c, v, c0, c0 + h, c0 + h, c0 + m, false))) return rc;
-    if ((rc = panel32(c, v, c0 + h, m - h, mode))) return rc;
-    PhaseTimer t(c, PH_PANEL);
-    K_TRY(launch_laswp_scale(v.a, v.ld, v.n, c0 + h, c0 + m, c->d_ipiv + v.goff, v.goff, c->mx->dinv + v.goff, c0,
-                             c0 + h, true, c->d_status, c->stream));
+    if ((rc = right_part32(c, v, c0, c0 + h, c0 + h, c0 + m, false, inner))) return rc;
+    if ((rc = panel32_rec(c, v, c0 + h, m - h, mode, left))) return rc;
+    left.add(c0 + h, c0 + m, c0, c0 + h);
     return 0;
+}
+
+static int panel32(lu2gpu_ctx *c, const View32 &v, int c0, int m, int mode)
+{
+    SwapJobs left;
+    const int rc = panel32_rec(c, v, c0, m, mode, left);
+    if (rc) return rc;
+    PhaseTimer t(c, PH_PANEL);
+    return swap_rows_now32(c, v, left);
 }
 
 // FP32 forward solve with the stored factors (what the factorization applies
@@ -2844,7 +2894,8 @@ static int factor32_or_fail(lu2gpu_ctx *c, int n, float *a, long ld, int nb, int
     }
     const cudaStream_t main_st = c->stream;
     const int all_ctas = c->leaf_ctas;
-    int rc = panel32(c, v, 0, std::min(nb, n), mode);  // the first panel, on the main stream
+    SwapJobs left;  // the factored panel's exchanges on its own columns, done with its right part's
+    int rc = panel32_rec(c, v, 0, std::min(nb, n), mode, left);  // the first panel, on the main stream
     for (int i = 0; rc == 0 && i < n; i += nb) {
         const int w = std::min(nb, n - i), i1 = i + w, w1 = std::min(nb, n - i1);
         if (i > 0 && cudaStreamWaitEvent(main_st, m->ev_panel, 0) != cudaSuccess) {
@@ -2858,14 +2909,15 @@ static int factor32_or_fail(lu2gpu_ctx *c, int n, float *a, long ld, int nb, int
             CU_TRY(cudaStreamWaitEvent(m->side, m->ev_cols, 0));
             c->stream = m->side;
             c->leaf_ctas = std::min(all_ctas, R);
-            const int r = panel32(c, v, i1, w1, mode);
+            left = SwapJobs();
+            const int r = panel32_rec(c, v, i1, w1, mode, left);
             c->stream = main_st;
             c->leaf_ctas = all_ctas;
             if (r) return r;
             CU_TRY(cudaEventRecord(m->ev_panel, m->side));
             return 0;
         };
-        rc = right_part32_split(c, v, i, i1, i1, n, w1, sms - R, next_panel);
+        rc = right_part32_split(c, v, i, i1, i1, n, w1, sms - R, left, next_panel);
     }
     c->stream = main_st;
     c->leaf_ctas = all_ctas;

@@ -170,6 +170,21 @@ cudaError_t launch_laswp_scale(double *a, long ld, int nrows, int k0, int k1, co
                                const double *dinv, int cs, int ce, bool scale, int *status, cudaStream_t st);
 cudaError_t launch_laswp_scale(float *a, long ld, int nrows, int k0, int k1, const int *ipiv, int goff,
                                const float *dinv, int cs, int ce, bool scale, int *status, cudaStream_t st);
+// Several of them in one launch, all with scaling: exchanges k0..k1-1 on
+// columns cs..ce-1 each.  No two jobs share a column.
+struct SwapJob {
+    int k0, k1, cs, ce;
+};
+constexpr int SWAP_JOBS = 8;  // a panel of 512 columns leaves 5 with 16-column leaves, and one more joins
+struct SwapJobs {
+    int n = 0;
+    SwapJob j[SWAP_JOBS];
+    void add(int k0, int k1, int cs, int ce) { j[n++] = SwapJob{k0, k1, cs, ce}; }
+};
+cudaError_t launch_laswp_jobs(double *a, long ld, int nrows, const SwapJobs &jobs, const int *ipiv, int goff,
+                              const double *dinv, int *status, cudaStream_t st);
+cudaError_t launch_laswp_jobs(float *a, long ld, int nrows, const SwapJobs &jobs, const int *ipiv, int goff,
+                              const float *dinv, int *status, cudaStream_t st);
 
 // In place X := T^{-1} X for the unit lower triangle T = strict lower part of
 // a[r0..r0+K)[r0..r0+K) and X = a[r0..r0+K)[cs..ce); also writes
