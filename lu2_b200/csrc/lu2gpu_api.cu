@@ -2140,6 +2140,12 @@ struct View32 {
 // Top-level right part of the precision forms with the trailing update in two
 // launches: columns cs..cs+w1-1 first (the next panel's), then `after_first()`
 // (the lookahead hook), then the rest; update kernels capped at max_ctas CTAs.
+// Each launch's columns of U12 are converted right before it.  The second
+// conversion, a few us of small CTAs, also lets the next panel's first leaf
+// onto the GPU before the update's CTAs: a leaf's cluster needs 16 free SMs side
+// by side, finds none once the persistent update lies on all parts of the GPU
+// (the panel then waited for the whole update), and leaves them free for the
+// panel's next leaves.
 template <typename Hook>
 static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, int cs, int ce, int w1, int max_ctas,
                               SwapJobs left, Hook after_first);
@@ -2213,7 +2219,7 @@ static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, in
         {
             PhaseTimer t(c, PH_DGEMM);
             K_TRY(launch_quant_fp8_tiles(L, v.ld, M, K, m->l8, K, dqa, c->stream));
-            K_TRY(launch_quant_fp8_tiles(m->bt32top, K, N, K, m->b8, K, dqb, c->stream));
+            K_TRY(launch_quant_fp8_tiles(m->bt32top, K, w1, K, m->b8, K, dqb, c->stream));
             K_TRY(launch_lowp_update_fp8(m->l8, K, dqa, m->b8, K, dqb, C, v.ld, M, w1, K, c->d_status, max_ctas,
                                          c->stream));
         }
@@ -2221,6 +2227,8 @@ static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, in
     if (rc) return rc;
         if (w1 < N) {
             PhaseTimer t(c, PH_DGEMM);
+            K_TRY(launch_quant_fp8_tiles(m->bt32top + (size_t)w1 * K, K, N - w1, K, m->b8 + (size_t)w1 * K, K,
+                                         dqb + (size_t)(w1 / 128) * KB, c->stream));
             K_TRY(launch_lowp_update_fp8(m->l8, K, dqa, m->b8 + (size_t)w1 * K, K, dqb + (size_t)(w1 / 128) * KB,
                                          C + w1, v.ld, M, N - w1, K, c->d_status, max_ctas, c->stream));
         }
@@ -2238,7 +2246,7 @@ static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, in
         K_TRY(launch_absmax2(L, v.ld, M, K, X, v.ld, K, N, m->amax(), c->stream));
         K_TRY(launch_panel_scales(m->amax(), m->scales(), c->stream));
         K_TRY(launch_f32_to_bf16(L, v.ld, m->l16, K, M, K, m->scales(), c->stream));
-        K_TRY(launch_f32_transpose_bf16(X, v.ld, K, N, m->u16, m->scales() + 1, c->stream));
+        K_TRY(launch_f32_transpose_bf16(X, v.ld, K, w1, m->u16, m->scales() + 1, c->stream));
         K_TRY(launch_lowp_update_bf16(m->l16, K, u16, K, C, v.ld, M, w1, K, m->scales() + 2, c->d_status, max_ctas,
                                       c->stream));
     }
@@ -2246,6 +2254,8 @@ static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, in
     if (rc) return rc;
     if (w1 < N) {
         PhaseTimer t(c, PH_DGEMM);
+        K_TRY(launch_f32_transpose_bf16(X + w1, v.ld, K, N - w1, static_cast<char *>(m->u16) + (size_t)w1 * K * 2,
+                                        m->scales() + 1, c->stream));
         K_TRY(launch_lowp_update_bf16(m->l16, K, u16 + (size_t)w1 * K * 2, K, C + w1, v.ld, M, N - w1, K,
                                       m->scales() + 2, c->d_status, max_ctas, c->stream));
     }
