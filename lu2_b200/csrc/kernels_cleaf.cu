@@ -1,6 +1,6 @@
 // kernels_cleaf.cu -- the panel leaf on one thread-block cluster: LU with
-// partial pivoting of a slab of up to 64 columns whose rows live in the
-// registers of at most 16 CTAs.
+// partial pivoting of a slab of up to 64 columns whose rows live in the shared
+// memory of at most 16 CTAs.
 //
 // Reference behaviour (telmin/lu2): column_decomposition, lu2tlib.c:1041-1066
 // inside the slab recursion lu2tlib.c:1095-1128; pivot search cblas_idamax
