@@ -464,8 +464,9 @@ __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafPara
         for (int jb = 0; jb < nbk; jb++) {
             const int ip = blk + jb, c = c0 + ip, par = ip & 1;
             if (!help) {
-                const bool use_ls = REF && ip > 0 &&
-                                    (mode == PIVOT_REF_FIRST || ((c + goff) & 1));  // lu2tlib.c:1052
+                // lu2tlib.c:1052, counted over the whole matrix; as in leaf_kernel the first
+                // column of each 16 searches itself (odd when a slab begins at an odd row)
+                const bool use_ls = REF && (ip & 15) && (mode == PIVOT_REF_FIRST || ((c + goff) & 1));
                 // this thread's candidate, the warp's, the CTA's
                 unsigned long long key = 0;
                 int kp = INT_MAX, kr = 0;
