@@ -328,12 +328,22 @@ __device__ void ir_solve(const float *F, int n, int fs, float *V, int r)
             for (int k = 0; k < 32; k++)
                 if (lane == k && k < bw) d = f[k];
             const float inv = 1.f / d;
+            // a subnormal pivot below 2^-128 has no FP32 reciprocal: such a block divides
+            const bool divide = __any_sync(0xffffffffu, isinf(inv));
             for (int q = warp; q < r; q += nw) {
                 float v = lane < bw ? V[(size_t)q * n + b0 + lane] : 0.f;
+                if (!divide) {
 #pragma unroll
-                for (int k = 0; k < 32; k++) {
-                    const float y = v * inv, yk = __shfl_sync(0xffffffffu, y, k);
-                    v = lane == k ? y : (lane > k ? fmaf(-f[k], yk, v) : v);
+                    for (int k = 0; k < 32; k++) {
+                        const float y = v * inv, yk = __shfl_sync(0xffffffffu, y, k);
+                        v = lane == k ? y : (lane > k ? fmaf(-f[k], yk, v) : v);
+                    }
+                } else {
+                    for (int k = 0; k < bw; k++) {
+                        const float yk = __shfl_sync(0xffffffffu, v, k) / __shfl_sync(0xffffffffu, d, k);
+                        if (lane == k) v = yk;
+                        if (lane > k && lane < bw) v = fmaf(-F[(size_t)(b0 + lane) * fs + b0 + k], yk, v);
+                    }
                 }
                 if (lane < bw) V[(size_t)q * n + b0 + lane] = v;
             }
