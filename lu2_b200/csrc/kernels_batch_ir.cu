@@ -3,7 +3,7 @@
 // until x is written into its b columns) is converted to FP32, factored in
 // FP32, and refined in FP64 -- r = b - A x from the FP64 matrix, the
 // correction solved with the FP32 factors -- until every right-hand side has
-// an HPL scaled residual below 16 (or max_iter corrections).
+// an HPL scaled residual below 16 however it is summed (or max_iter corrections).
 //
 // Factor storage follows lu2's elimination (lu2.c:541-554, lu2tlib.c:1057-
 // 1059): the pivot row is scaled by 1/pivot right of the diagonal (a unit
@@ -491,6 +491,11 @@ batch_ir_kernel(double *data, const BatchSys *sys, const long long *woff, uint8_
             for (int idx = tid; idx < n * r; idx += T) X[idx] = 0.0;
             __syncthreads();
             ir_residual(A, S.ld, n, r, X, R, true, s_red, s_rmax, s_xmax, s_bmax, &s_anorm);
+            // lu2's bar of 16 with room for the rounding of a residual: summed in any order
+            // it is off by at most (n + 1) u (|A||x| + |b|), (n + 1) / n in units of h, here
+            // and where the caller sums it (held to 16 itself, 1 of 20,000 systems came back
+            // at 16.01)
+            const double bar = 16.0 - 2.0 * (n + 1) / n;
             for (it = 1; it <= max_iter; it++) {
                 for (int i = tid; i < n; i += T) {
                     const int from = perm[i];
@@ -504,7 +509,7 @@ batch_ir_kernel(double *data, const BatchSys *sys, const long long *woff, uint8_
                     bool ok = true;
                     for (int q = 0; q < r; q++) {
                         const double h = s_rmax[q] / (1.1102230246251565e-16 * (s_anorm * s_xmax[q] + s_bmax[q]) * n);
-                        if (!(h < 16.0)) ok = false;
+                        if (!(h < bar)) ok = false;
                     }
                     s_done = ok;
                 }
