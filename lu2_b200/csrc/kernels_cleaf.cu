@@ -614,7 +614,8 @@ __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafPara
         if (tid < ((rem + 7) & ~7)) {
             const int col = blk + CL_B + tid;
             const T dl = sh.d[blk + (lane & (CL_B - 1))], il = cl_zero(dl) ? T(1) : T(1) / dl;
-            const unsigned mates = __activemask();
+            const int lanes = min(32, ((rem + 7) & ~7) - 32 * warp);  // of this warp in here, from lane 0 on
+            const unsigned mates = 0xffffffffu >> (32 - lanes);
             T x[CL_B], lij[CL_B][CL_B];
 #pragma unroll
             for (int j = 0; j < CL_B; j++) {

@@ -51,3 +51,27 @@ def test_reference_search_in_slabs_at_any_row(rows, m, start):
     a = np.random.default_rng(rows + start).uniform(-0.5, 0.5, (rows, m))
     a[np.arange(m), np.arange(m)] += m  # its odd columns' pivots need not be large: keep the growth small
     np.testing.assert_array_equal(gpu_pivots(a, start), reference_pivots(a, start))
+
+
+@pytest.mark.parametrize("m", [9, 15, 17, 31, 40, 41, 48, 63])
+@pytest.mark.parametrize("rows", [100, 700])
+def test_pivot_rows_right_of_a_block(rows, m):
+    """The 8 pivot rows of a block are finished one column per thread: widths that fill
+    part of the first warp, all of it, and part of the second.  Backward error as
+    Higham, Theorem 9.3: |P A - L U| <= (m + 4) u |L| |U|, with as much again for the
+    check's own product."""
+    a = np.random.default_rng(rows + m).uniform(-0.5, 0.5, (rows, m))
+    slab = np.ascontiguousarray(a.T)
+    pv = np.zeros(m, dtype=np.int32)
+    L.load().cm_column_decomposition_recursive(rows, slab.ctypes.data, m, pv.ctypes.data, 0)
+    f = slab.T.copy()
+    for k, p in enumerate(pv):
+        a[[k, p]] = a[[p, k]]
+    d = f[np.arange(m), np.arange(m)]
+    low = np.tril(f)
+    low[np.arange(m), np.arange(m)] = 1.0
+    low[:m] *= d[:, None]  # pivot rows are scaled by 1/pivot as a whole
+    up = np.triu(f[:m], 1) + np.eye(m)
+    bar = 2 * (m + 4) * 2.0 ** -53 * (np.abs(low) @ np.abs(up))
+    assert np.all(np.abs(a - low @ up) <= bar)
+    assert np.all(np.abs(f[m:]) <= np.abs(d))
