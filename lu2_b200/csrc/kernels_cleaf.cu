@@ -47,7 +47,8 @@
 //
 // Every wait is bounded: when one gives up, the CTA records the error and
 // leaves the loop at its next barrier; the others find the error word and do
-// the same.  No CTA exits before all have arrived at the last cluster barrier.
+// the same.  No CTA exits before all have arrived at the last cluster barrier,
+// and one that gave up stays a little longer, for what is still on its way to it.
 #include <atomic>
 #include <climits>
 
@@ -72,6 +73,7 @@ constexpr int CL_HELP = 128;  // helpers: store and send the decided rows beside
 constexpr int CL_ALL = CL_TPB + CL_HELP;
 constexpr int CL_B = 8;      // columns of a block
 constexpr int CL_MAXC = 16;  // CTAs of a cluster
+constexpr unsigned long long CL_LINGER_NS = 50000;  // that a CTA stays after a failed wait
 
 template <typename T, int W, int RT>
 struct CLeafCfg {
@@ -692,6 +694,14 @@ __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafPara
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // a CTA that gave up has not waited for all that was sent to it, and the barrier
+    // does not order st.async: its shared memory stays until the last of it has landed
+    // (all was sent before the barrier; 16 CTAs' messages take 0.6 us)
+    if (CL > 1 && sh.fail) {
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < CL_LINGER_NS) {
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
