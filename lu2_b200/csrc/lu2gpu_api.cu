@@ -927,6 +927,11 @@ extern "C" int lu2gpu_dgemm_dev(lu2gpu_ctx *c, int m, int n, int k, double alpha
         return LU2GPU_ERR_ARG;
     }
     if (m == 0 || n == 0) return 0;
+    // rows of A shorter than k (a single row may leave its stride zero)
+    if (k > 0 && (!a || !b || (lda < k && !(m == 1 && lda == 0)))) {
+        set_error("lu2gpu_dgemm_dev: A or B missing, or lda=%ld below k=%d", lda, k);
+        return LU2GPU_ERR_ARG;
+    }
     DeviceGuard g(c->device);
     int rc = begin_status(c);
     if (rc) return rc;
@@ -935,7 +940,7 @@ extern "C" int lu2gpu_dgemm_dev(lu2gpu_ctx *c, int m, int n, int k, double alpha
     const long ldx = ldy;
     const auto first = [](const double *p) { return reinterpret_cast<uintptr_t>(p); };
     const auto last = [&](const double *p, long ld, int cols) { return first(p) + ((size_t)(m - 1) * ld + cols) * 8; };
-    const bool in_place = k > 0 && !(lda & 1) && !(first(a) & 15) &&
+    const bool in_place = k > 0 && lda >= k && !(lda & 1) && !(first(a) & 15) &&
                           (last(a, lda, k) <= first(cm) || last(cm, ldc, n) <= first(a));
     double *y, *x = nullptr;
     if ((rc = stage(c, 0, (size_t)n * ldy, &y))) return rc;
