@@ -611,13 +611,11 @@ __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafPara
         __syncthreads();
         if (sh.fail) break;
         if (rem <= 0) break;  // the last block
-        // the 8 pivot rows right of the block, one column per thread (zeros past
-        // w; whole groups of 8 lanes, whose lanes hold the reciprocals)
-        if (tid < ((rem + 7) & ~7)) {
+        // the 8 pivot rows right of the block, one column per thread (zeros past w, in
+        // whole groups of 8), in whole warps: lanes 0..7 hold the reciprocals
+        if (warp * 32 < rem) {
             const int col = blk + CL_B + tid;
             const T dl = sh.d[blk + (lane & (CL_B - 1))], il = cl_zero(dl) ? T(1) : T(1) / dl;
-            const int lanes = min(32, ((rem + 7) & ~7) - 32 * warp);  // of this warp in here, from lane 0 on
-            const unsigned mates = 0xffffffffu >> (32 - lanes);
             T x[CL_B], lij[CL_B][CL_B];
 #pragma unroll
             for (int j = 0; j < CL_B; j++) {
@@ -637,10 +635,10 @@ __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafPara
                 T v = x[j];
 #pragma unroll
                 for (int i = 0; i < j; i++) v = cl_fnma(lij[j][i], x[i], v);
-                v *= __shfl_sync(mates, il, j);
+                v *= __shfl_sync(0xffffffffu, il, j);
                 if (rank == 0 && tid < rem) P.a[(size_t)(c0 + blk + j) * P.ld + c0 + col] = v;
-                x[j] = cl_zero(__shfl_sync(mates, dl, j)) ? T(0) : v;  // a zero pivot's column subtracts nothing
-                cl_st1(ub + (j * C::UP + tid) * ES, x[j]);
+                x[j] = cl_zero(__shfl_sync(0xffffffffu, dl, j)) ? T(0) : v;  // a zero pivot's column subtracts nothing
+                if (tid < ((rem + 7) & ~7)) cl_st1(ub + (j * C::UP + tid) * ES, x[j]);
             }
         }
         __syncthreads();
