@@ -721,15 +721,23 @@ static constexpr int cl_rows()
     return CL_MAXC * CLeafPick<T, W, TALL>::ROWS;
 }
 
-// shared memory and cluster size limits of one instance; true when a cluster of 16 can be resident
+// shared memory and cluster size limits of one instance, in the current context
+template <typename T, int W, bool TALL, bool REF>
+static cudaError_t cl_attributes()
+{
+    using C = CLeafPick<T, W, TALL>;
+    auto kern = cluster_leaf_kernel<T, W, C::ROWS / CL_TPB, REF>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+
+// true when a cluster of 16 of this instance can be resident
 template <typename T, int W, bool TALL, bool REF>
 static bool cl_prepare_1()
 {
     using C = CLeafPick<T, W, TALL>;
     auto kern = cluster_leaf_kernel<T, W, C::ROWS / CL_TPB, REF>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-        return false;
+    if (cl_attributes<T, W, TALL, REF>() != cudaSuccess) return false;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(16);
     cfg.blockDim = dim3(CL_ALL);
@@ -793,8 +801,8 @@ int leaf_width(int rows, size_t tsize, int max_ctas)
     return k > 16 ? k : 16;
 }
 
-template <typename T, int W, bool TALL = false>
-static cudaError_t cl_launch_w(CLeafParams<T> P, cudaStream_t st)
+template <typename T, int W, bool TALL, bool REF>
+static cudaError_t cl_launch_1(CLeafParams<T> P, cudaStream_t st)
 {
     using C = CLeafPick<T, W, TALL>;
     const int rows = P.n - P.c0;
@@ -802,6 +810,10 @@ static cudaError_t cl_launch_w(CLeafParams<T> P, cudaStream_t st)
     while (cl < 16 && cl * C::ROWS < rows) cl *= 2;
     P.rpc = (rows + cl - 1) / cl;
     if (P.rpc > C::ROWS) return cudaErrorInvalidConfiguration;
+    // set for every launch, as they belong to the CUDA context and not to the
+    // device: they are gone after cudaDeviceReset
+    const cudaError_t e = cl_attributes<T, W, TALL, REF>();
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)cl);
     cfg.blockDim = dim3(CL_ALL);
@@ -813,8 +825,13 @@ static cudaError_t cl_launch_w(CLeafParams<T> P, cudaStream_t st)
     cfg.attrs = at;
     cfg.numAttrs = 1;
     count_launch();
-    return P.mode == PIVOT_PARTIAL ? cudaLaunchKernelEx(&cfg, cluster_leaf_kernel<T, W, C::ROWS / CL_TPB, false>, P)
-                                   : cudaLaunchKernelEx(&cfg, cluster_leaf_kernel<T, W, C::ROWS / CL_TPB, true>, P);
+    return cudaLaunchKernelEx(&cfg, cluster_leaf_kernel<T, W, C::ROWS / CL_TPB, REF>, P);
+}
+
+template <typename T, int W, bool TALL = false>
+static cudaError_t cl_launch_w(const CLeafParams<T> &P, cudaStream_t st)
+{
+    return P.mode == PIVOT_PARTIAL ? cl_launch_1<T, W, TALL, false>(P, st) : cl_launch_1<T, W, TALL, true>(P, st);
 }
 
 template <typename T>

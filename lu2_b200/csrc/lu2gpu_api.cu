@@ -1944,11 +1944,10 @@ constexpr size_t NOALLOC_SCRATCH_BYTES = NA_BT + na_round(NA_BT_BYTES);  // abou
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
 
-// Device address of g_noalloc_scratch per device, looked up once per device
-// with that device current.  In host code the symbol itself is only a host-side
-// stand-in and must never be passed to a kernel.
+// In host code the symbol itself is only a host-side stand-in and must never be
+// passed to a kernel: noalloc_setup asks for its device address, with the device
+// current.
 static std::mutex g_noalloc_mu;
-static void *g_noalloc_ptr[128];
 static int g_noalloc_ctas[128];
 static int g_noalloc_major[128];  // compute capability major of each device, 0 until looked up
 // leaf publication stamps per device; the slots start zeroed (static storage)
@@ -1976,20 +1975,21 @@ static int noalloc_setup(int device, unsigned char **base, int *leaf_ctas)
                   g_noalloc_major[device]);
         return LU2GPU_ERR_NODEV;
     }
-    if (!g_noalloc_ptr[device]) {
-        void *p = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-        if (e != cudaSuccess || !p) {
-            cudaGetLastError();
-            set_error("lu2gpu_lusolve_noalloc: cudaGetSymbolAddress failed on device %d: %s", device,
-                      cudaGetErrorString(e));
-            return LU2GPU_ERR_CUDA;
-        }
-        int ctas = leaf_max_ctas(device);
-        g_noalloc_ctas[device] = ctas < NOALLOC_LEAF_CTAS ? ctas : NOALLOC_LEAF_CTAS;
-        g_noalloc_ptr[device] = p;
+    // asked for in every call: it belongs to the CUDA context, which a program may
+    // end (cudaDeviceReset) and begin again
+    void *p = nullptr;
+    const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+    if (e != cudaSuccess || !p) {
+        cudaGetLastError();
+        set_error("lu2gpu_lusolve_noalloc: cudaGetSymbolAddress failed on device %d: %s", device,
+                  cudaGetErrorString(e));
+        return LU2GPU_ERR_CUDA;
     }
-    *base = (unsigned char *)g_noalloc_ptr[device];
+    if (!g_noalloc_ctas[device]) {
+        const int ctas = leaf_max_ctas(device);
+        g_noalloc_ctas[device] = ctas < NOALLOC_LEAF_CTAS ? ctas : NOALLOC_LEAF_CTAS;
+    }
+    *base = (unsigned char *)p;
     *leaf_ctas = g_noalloc_ctas[device];
     return 0;
 }
