@@ -545,6 +545,17 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParam
     }
 }
 
+// CTAs of a solve of nblk blocks, and the shared memory of one
+static int ts_grid(int nblk, int sms) { return nblk < sms ? nblk : sms; }
+static size_t ts_bytes(int nblk, int sms, bool lower, int nr, size_t tsize)
+{
+    const int G = ts_grid(nblk, sms), own = (nblk + G - 1) / G;
+    return ((size_t)TS_B * TS_TLD + 2 * TS_XQ * nr + (nr == 8 && !lower ? TS_B * nr : 0) +
+            (size_t)own * TS_B * (nr + (lower ? 1 : 0))) *
+           tsize;
+}
+constexpr size_t TS_SMEM_MAX = 220 * 1024;
+
 template <typename T, bool LOWER, int NR>
 static cudaError_t ts_launch(TriParams<T> P, cudaStream_t st, bool *used)
 {
@@ -553,13 +564,12 @@ static cudaError_t ts_launch(TriParams<T> P, cudaStream_t st, bool *used)
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    const int G = P.nblk < sms ? P.nblk : sms, own = (P.nblk + G - 1) / G;
-    const size_t smem = ((size_t)TS_B * TS_TLD + 2 * TS_XQ * NR + (NR == 8 && !LOWER ? TS_B * NR : 0) +
-                         (size_t)own * TS_B * (NR + (LOWER ? 1 : 0))) *
-                        sizeof(T);
-    if (smem > 220 * 1024) return cudaSuccess;  // too many blocks per CTA: the caller's other way
+    const int G = ts_grid(P.nblk, sms);
+    const size_t smem = ts_bytes(P.nblk, sms, LOWER, NR, sizeof(T));
+    if (smem > TS_SMEM_MAX) return cudaSuccess;  // too many blocks per CTA: the caller's other way
     auto kern = tri_solve_kernel<T, LOWER, NR>;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_MAX)) != cudaSuccess)
+        return e;
     void *args[] = {&P};
     count_launch();
     e = cudaLaunchCooperativeKernel((const void *)kern, dim3(G), dim3(TS_THREADS), args, smem, st);
@@ -623,6 +633,24 @@ cudaError_t launch_upper_solve(const float *a, long ld, int n, int nrhs, const f
     return upper_t(a, ld, n, nrhs, y, ldy, x, ldx, bs, st, used);
 }
 
+// blocks of the lower solve: every panel of nb rows in blocks of its own
+static int lower_blocks(int n, int nb)
+{
+    const int npan = (n + nb - 1) / nb, last = n - (npan - 1) * nb;
+    return (npan - 1) * ((nb + TS_B - 1) / TS_B) + (last + TS_B - 1) / TS_B;
+}
+
+bool tri_solves_fit(int n, int nb, size_t tsize)
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+        return false;
+    const int nr = tsize == sizeof(double) ? ts_maxr<double>() : ts_maxr<float>();
+    return ts_bytes(lower_blocks(n, nb), sms, true, nr, tsize) <= TS_SMEM_MAX &&
+           ts_bytes((n + TS_B - 1) / TS_B, sms, false, nr, tsize) <= TS_SMEM_MAX;
+}
+
 template <typename T>
 static cudaError_t lower_t(const T *a, long ld, int n, int nb, const int *rows, const T *dinv, const T *b, long ldb,
                            int nrhs, T *y, long ldy, const BsBuffers &bs, cudaStream_t st, bool *used)
@@ -635,8 +663,7 @@ static cudaError_t lower_t(const T *a, long ld, int n, int nb, const int *rows, 
     P.n = n;
     P.nb = nb;
     P.bpp = (nb + TS_B - 1) / TS_B;
-    const int npan = (n + nb - 1) / nb, last = n - (npan - 1) * nb;
-    P.nblk = (npan - 1) * P.bpp + (last + TS_B - 1) / TS_B;
+    P.nblk = lower_blocks(n, nb);
     P.y = b;
     P.ldy = ldb;
     P.x = y;

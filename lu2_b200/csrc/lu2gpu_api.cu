@@ -175,29 +175,38 @@ struct DeviceGuard {
     }
 };
 
-static int grow(void **p, size_t *cap, size_t bytes)
+// false, without a message, where the memory cannot be had: the caller has another way
+static bool try_grow(void **p, size_t *cap, size_t bytes)
 {
-    if (*cap >= bytes && *p) return 0;
+    if (*cap >= bytes && *p) return true;
     if (*p) cudaFree(*p);
     *p = nullptr;
     *cap = 0;
     if (cudaMalloc(p, bytes) != cudaSuccess) {
         cudaGetLastError();
-        set_error("cudaMalloc of %zu bytes failed", bytes);
-        return LU2GPU_ERR_NOMEM;
+        return false;
     }
     *cap = bytes;
-    return 0;
+    return true;
+}
+
+static int grow(void **p, size_t *cap, size_t bytes)
+{
+    if (try_grow(p, cap, bytes)) return 0;
+    set_error("cudaMalloc of %zu bytes failed", bytes);
+    return LU2GPU_ERR_NOMEM;
 }
 
 // The persistent forward solve's map for the pivots ipiv (device) and panel
-// width nb, enqueued; null where its buffers cannot be had (the solve then
-// goes panel by panel).
-static const int *solve_rows(lu2gpu_ctx *c, int n, int nb, const int *ipiv)
+// width nb of factors with elements of tsize bytes, enqueued; null where the
+// solves do not fit or their buffers cannot be had (the solve then goes panel by
+// panel).
+static const int *solve_rows(lu2gpu_ctx *c, int n, int nb, size_t tsize, const int *ipiv)
 {
+    if (!tri_solves_fit(n, nb, tsize)) return nullptr;
     const size_t each = ((size_t)n + nb - 1) / nb * n;
-    if (!bs_buffers(c, n) || grow((void **)&c->d_plan, &c->plan_cap, 2 * each * sizeof(int)) ||
-        grow((void **)&c->d_fwd, &c->fwd_cap, (size_t)n * BS_MAXR * sizeof(double)) ||
+    if (!bs_buffers(c, n) || !try_grow((void **)&c->d_plan, &c->plan_cap, 2 * each * sizeof(int)) ||
+        !try_grow((void **)&c->d_fwd, &c->fwd_cap, (size_t)n * BS_MAXR * sizeof(double)) ||
         launch_solve_plan(ipiv, n, nb, c->d_plan + each, c->d_plan, c->d_status, c->stream) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
@@ -869,7 +878,7 @@ extern "C" int lu2gpu_solve(lu2gpu_ctx *c, int n, const double *a, long lda, int
     if ((rc = ensure_work(c, n, nrhs, nb))) return rc;
     if ((rc = begin_status(c))) return rc;
     K_TRY(launch_diag_inv(a, lda, n, c->d_dinv, c->stream));
-    const int *rows = nrhs <= SOLVE_FEW_RHS ? solve_rows(c, n, nb, ipiv) : nullptr;
+    const int *rows = nrhs <= SOLVE_FEW_RHS ? solve_rows(c, n, nb, sizeof(double), ipiv) : nullptr;
     if (rows) {
         bool used = false;
         for (int q = 0; q < nrhs; q += BS_MAXR) {
@@ -2983,7 +2992,7 @@ extern "C" int lu2gpu_mixed_solve(lu2gpu_ctx *c, int n, const double *a, long ld
     if ((rc = factor32_or_fail(c, n, m->a32, ld32, nb, pivot_mode))) return rc;
     CU_TRY(cudaEventRecord(ev[1], c->stream));
 
-    const int *rows = solve_rows(c, n, nb, c->d_ipiv);
+    const int *rows = solve_rows(c, n, nb, sizeof(float), c->d_ipiv);
     // refinement: x_0 = 0, r_0 = b; d = LU^{-1} r (FP32), x += d, r = b - A x (FP64)
     CU_TRY(cudaMemsetAsync(x, 0, (size_t)n * sizeof(double), c->stream));
     CU_TRY(cudaMemcpyAsync(r, b, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
@@ -3129,7 +3138,7 @@ extern "C" int lu2gpu_gmres_solve(lu2gpu_ctx *c, int n, const double *a, long ld
     if ((rc = factor32_or_fail(c, n, m->a32, ld32, nb, LU2GPU_PIVOT_PARTIAL))) return rc;
     CU_TRY(cudaEventRecord(ev[1], c->stream));
 
-    const int *rows = solve_rows(c, n, nb, c->d_ipiv);
+    const int *rows = solve_rows(c, n, nb, sizeof(float), c->d_ipiv);
     const double one = 1.0;
     CU_TRY(cudaMemcpyAsync(dots + 128, &one, sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CU_TRY(cudaMemsetAsync(x, 0, (size_t)n * sizeof(double), c->stream));

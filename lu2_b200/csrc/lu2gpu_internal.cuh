@@ -246,6 +246,8 @@ cudaError_t launch_lower_solve(const double *a, long ld, int n, int nb, const in
 cudaError_t launch_lower_solve(const float *a, long ld, int n, int nb, const int *rows, const float *dinv,
                                const float *b, long ldb, int nrhs, float *y, long ldy, const BsBuffers &bs,
                                cudaStream_t st, bool *used);
+// whether both fit for factors of panel width nb (elements of tsize bytes)
+bool tri_solves_fit(int n, int nb, size_t tsize);
 // rows[P][f] (P < ceil(n / nb)): the position, before panel P's exchanges, of
 // the row that ends at position f >= P nb of the whole sequence ipiv (0-based,
 // row k exchanged with ipiv[k] >= k).  inv: scratch of the same size.  A pivot
