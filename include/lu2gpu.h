@@ -185,7 +185,11 @@ int lu2gpu_backsolve(lu2gpu_ctx *ctx, int n, int nrhs, const double *a, long lda
  * augmented columns (pivots with 1/pivot scaling, unit-lower solve, update of
  * the rows below; lu2.c:524-581), then the back substitution.  lu2 itself
  * keeps only the last panel's pivots and cannot do this.  b (device, n x nrhs,
- * row stride ldb) is overwritten by x.  a is not modified. */
+ * row stride ldb) is overwritten by x.  a is not modified.  The context keeps
+ * what the solve needs beside the factors until it is destroyed: row maps of
+ * 4 n (n / nb + 1) bytes (1 / (2 nb) of the matrix) and a few hundred bytes per
+ * row; so do the precision forms below.  Where that memory cannot be had the
+ * solve goes panel by panel. */
 int lu2gpu_solve(lu2gpu_ctx *ctx, int n, const double *a, long lda, int nb, const int *ipiv, double *b, long ldb,
                  int nrhs);
 

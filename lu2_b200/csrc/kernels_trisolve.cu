@@ -70,7 +70,7 @@ struct TriParams {
     T *x;
     long ldx;
     int nr;
-    const int *rows;  // lower: [panel][n] positions before each panel, by final position
+    const int *rows;  // lower: positions before each panel, by final position (solve_map_at)
     const T *dinv;    // lower: 1/pivot
     unsigned long long *xslots;  // element (row, q) at 2 (row BS_MAXR + q)
     unsigned epoch;
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParam
             else if (!LOWER || panel_of(p) == panel_of(p_src))
                 row[h] = r;
             else
-                row[h] = __ldg(P.rows + (size_t)(panel_of(p_src) + 1) * P.n + r);  // its position after the source's panel
+                row[h] = __ldg(P.rows + solve_map_at(panel_of(p_src) + 1, P.n, P.nb) + r);  // after the source's panel
         }
     };
     const bool vec = ((reinterpret_cast<uintptr_t>(P.a) & (2 * sizeof(T) - 1)) == 0) && ((P.ld & 1) == 0) &&

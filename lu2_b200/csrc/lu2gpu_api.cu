@@ -125,7 +125,7 @@ struct lu2gpu_ctx {
     int bsx_cap = 0;  // rows
     unsigned bs_epoch = 0;
     BsBuffers bs{};
-    // the forward solve with stored factors: row maps (two [panels][n] arrays), transformed right-hand sides
+    // the forward solve with stored factors: row map and its scratch, transformed right-hand sides
     int *d_plan = nullptr;
     size_t plan_cap = 0;
     double *d_fwd = nullptr;
@@ -200,14 +200,15 @@ static int grow(void **p, size_t *cap, size_t bytes)
 // The persistent forward solve's map for the pivots ipiv (device) and panel
 // width nb of factors with elements of tsize bytes, enqueued; null where the
 // solves do not fit or their buffers cannot be had (the solve then goes panel by
-// panel).
+// panel).  Kept until the context is destroyed: with its scratch 4 n (n / nb + 1)
+// bytes, 1 / (2 nb) of an FP64 matrix.
 static const int *solve_rows(lu2gpu_ctx *c, int n, int nb, size_t tsize, const int *ipiv)
 {
     if (!tri_solves_fit(n, nb, tsize)) return nullptr;
-    const size_t each = ((size_t)n + nb - 1) / nb * n;
-    if (!bs_buffers(c, n) || !try_grow((void **)&c->d_plan, &c->plan_cap, 2 * each * sizeof(int)) ||
+    const size_t map = solve_map_ints(n, nb);
+    if (!bs_buffers(c, n) || !try_grow((void **)&c->d_plan, &c->plan_cap, 2 * map * sizeof(int)) ||
         !try_grow((void **)&c->d_fwd, &c->fwd_cap, (size_t)n * BS_MAXR * sizeof(double)) ||
-        launch_solve_plan(ipiv, n, nb, c->d_plan + each, c->d_plan, c->d_status, c->stream) != cudaSuccess) {
+        launch_solve_plan(ipiv, n, nb, c->d_plan + map, c->d_plan, c->d_status, c->stream) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }

@@ -248,10 +248,20 @@ cudaError_t launch_lower_solve(const float *a, long ld, int n, int nb, const int
                                cudaStream_t st, bool *used);
 // whether both fit for factors of panel width nb (elements of tsize bytes)
 bool tri_solves_fit(int n, int nb, size_t tsize);
-// rows[P][f] (P < ceil(n / nb)): the position, before panel P's exchanges, of
-// the row that ends at position f >= P nb of the whole sequence ipiv (0-based,
-// row k exchanged with ipiv[k] >= k).  inv: scratch of the same size.  A pivot
-// outside [k, n) sets ERR_BAD_ARG in status[1].
+// rows[solve_map_at(P) + f] (P < ceil(n / nb)): the position, before panel P's
+// exchanges, of the row that ends at position f >= P nb of the whole sequence
+// ipiv (0-based, row k exchanged with ipiv[k] >= k).  inv: scratch of the same
+// size, solve_map_ints(n, nb).  A pivot outside [k, n) sets ERR_BAD_ARG in
+// status[1].
+__host__ __device__ inline size_t solve_map_at(int P, int n, int nb)
+{
+    return (size_t)P * n - (size_t)nb * P * (P + 1) / 2;
+}
+inline size_t solve_map_ints(int n, int nb)
+{
+    const size_t npan = ((size_t)n + nb - 1) / nb;
+    return npan * n - nb * npan * (npan - 1) / 2;
+}
 cudaError_t launch_solve_plan(const int *ipiv, int n, int nb, int *inv, int *rows, int *status, cudaStream_t st);
 
 // out[k] = 1 / a[k][k] (1 for an exactly zero pivot)
