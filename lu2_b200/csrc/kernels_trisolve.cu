@@ -640,12 +640,40 @@ static int lower_blocks(int n, int nb)
     return (npan - 1) * ((nb + TS_B - 1) / TS_B) + (last + TS_B - 1) / TS_B;
 }
 
-bool tri_solves_fit(int n, int nb, size_t tsize)
+static int ts_sms()
 {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-        return false;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return sms;
+}
+
+// Right-hand sides (FP64) up to which the two persistent solves beat the panel
+// loop.  A pass of 8 walks the chain of blocks again; the loop's panels cost about
+// the same for any of these numbers.  us, persistent / panel loop:
+//   one block (n = 100, panels of 128):  8: 73 / 68, 16: 104 / 82; of 16:  16: 152 / 163, 24: 207 / 178
+//   panels of 512, n = 4096:  32: 3293 / 3779 (the loop's block solves are slow there)
+//   256:  17: 2044 / 1975 (n = 40000: 20.6 / 21.8 ms), 24: 2463 / 2167
+//   128:  17: 2034 / 2115, 24: 2452 / 2279;  64:  17: 2361 / 2427, 24: 2814 / 2636
+//   48:  16: 2197 / 2408, 17: 2743 / 2596
+//   32:  24: 3313 / 3567, 25: 3984 / 3747; n = 37000, 8 blocks per CTA:  9: 34.5 / 28.1 ms
+//   16, n = 2048, one block per CTA:  24: 2648 / 2499-2717, 25: 3200 / 2764; n = 6144, 3:  16: 6054 / 6926,
+//       17: 8497 / 7489; n = 10240, 5:  8: 6.2 / 10.6, 9: 11.6 / 11.1-12.1 ms
+// (a block is never larger than a panel, and one of 16 rows costs a tile of 128)
+int tri_solve_few_rhs(int n, int nb)
+{
+    if (n <= TS_B) return nb >= 48 ? BS_MAXR : 16;
+    if (nb > 256) return 32;
+    if (nb >= 48) return nb >= 64 ? 18 : 16;
+    const int sms = ts_sms(), own = sms > 0 ? (lower_blocks(n, nb) + sms - 1) / sms : 1;
+    return own > 4 ? BS_MAXR : nb == 32 || own <= 2 ? 24 : 16;
+}
+
+bool tri_solves_fit(int n, int nb, size_t tsize)
+{
+    const int sms = ts_sms();
+    if (sms <= 0) return false;
     const int nr = tsize == sizeof(double) ? ts_maxr<double>() : ts_maxr<float>();
     return ts_bytes(lower_blocks(n, nb), sms, true, nr, tsize) <= TS_SMEM_MAX &&
            ts_bytes((n + TS_B - 1) / TS_B, sms, false, nr, tsize) <= TS_SMEM_MAX;

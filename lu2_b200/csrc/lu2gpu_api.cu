@@ -861,10 +861,8 @@ extern "C" int lu2gpu_lusolve(lu2gpu_ctx *c, int n, int nrhs, double *a, long ld
 // unit-lower solve and the update of the rows below -- what the factorization
 // does to its augmented columns (lu2.c:524-581) -- then the back substitution
 // (lu2.c:110-116).  b (n x nrhs, row stride ldb) is overwritten by x.
-// Up to SOLVE_FEW_RHS right-hand sides go through the two persistent solves,
-// eight at a time; more through one panel loop whose products take them all.
-constexpr int SOLVE_FEW_RHS = 32;
-
+// Few right-hand sides go through the two persistent solves, eight at a time;
+// more through one panel loop whose products take them all.
 extern "C" int lu2gpu_solve(lu2gpu_ctx *c, int n, const double *a, long lda, int nb, const int *ipiv, double *b,
                             long ldb, int nrhs)
 {
@@ -879,7 +877,7 @@ extern "C" int lu2gpu_solve(lu2gpu_ctx *c, int n, const double *a, long lda, int
     if ((rc = ensure_work(c, n, nrhs, nb))) return rc;
     if ((rc = begin_status(c))) return rc;
     K_TRY(launch_diag_inv(a, lda, n, c->d_dinv, c->stream));
-    const int *rows = nrhs <= SOLVE_FEW_RHS ? solve_rows(c, n, nb, sizeof(double), ipiv) : nullptr;
+    const int *rows = nrhs <= tri_solve_few_rhs(n, nb) ? solve_rows(c, n, nb, sizeof(double), ipiv) : nullptr;
     if (rows) {
         bool used = false;
         for (int q = 0; q < nrhs; q += BS_MAXR) {

@@ -248,6 +248,8 @@ cudaError_t launch_lower_solve(const float *a, long ld, int n, int nb, const int
                                cudaStream_t st, bool *used);
 // whether both fit for factors of panel width nb (elements of tsize bytes)
 bool tri_solves_fit(int n, int nb, size_t tsize);
+// right-hand sides up to which they are the faster way for FP64 factors
+int tri_solve_few_rhs(int n, int nb);
 // rows[solve_map_at(P) + f] (P < ceil(n / nb)): the position, before panel P's
 // exchanges, of the row that ends at position f >= P nb of the whole sequence
 // ipiv (0-based, row k exchanged with ipiv[k] >= k).  inv: scratch of the same
