@@ -325,6 +325,7 @@ static cudaError_t launch_laswp_t(T *a, long ld, int nrows, const SwapJobs &all,
                                   const T *dinv, bool scale, int *status, cudaStream_t st)
 {
     constexpr int VW = 16 / (int)sizeof(T);
+    if (all.n > SWAP_JOBS) return cudaErrorInvalidValue;
     SwapJobs jobs;
     // 16-byte accesses when every row segment starts on a 16-byte boundary
     bool vec = (reinterpret_cast<uintptr_t>(a) & 15) == 0 && ld % VW == 0;

@@ -175,11 +175,18 @@ cudaError_t launch_laswp_scale(float *a, long ld, int nrows, int k0, int k1, con
 struct SwapJob {
     int k0, k1, cs, ce;
 };
-constexpr int SWAP_JOBS = 8;  // a panel of 512 columns leaves 5 with 16-column leaves, and one more joins
+// A panel of m columns leaves one job per halving of its right part: 5 for 512
+// columns with 16-column leaves, 6 for the 1024 that lu2's panel calls take (their
+// halves are the widest exchange a launch does); one more joins.
+constexpr int SWAP_JOBS = 8;
 struct SwapJobs {
-    int n = 0;
+    int n = 0;  // beyond SWAP_JOBS: a job found no place, and the launch refuses all of them
     SwapJob j[SWAP_JOBS];
-    void add(int k0, int k1, int cs, int ce) { j[n++] = SwapJob{k0, k1, cs, ce}; }
+    void add(int k0, int k1, int cs, int ce)
+    {
+        if (n < SWAP_JOBS) j[n] = SwapJob{k0, k1, cs, ce};
+        if (n <= SWAP_JOBS) n++;
+    }
 };
 cudaError_t launch_laswp_jobs(double *a, long ld, int nrows, const SwapJobs &jobs, const int *ipiv, int goff,
                               const double *dinv, int *status, cudaStream_t st);
