@@ -611,9 +611,10 @@ __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafPara
         __syncthreads();
         if (sh.fail) break;
         if (rem <= 0) break;  // the last block
-        // the 8 pivot rows right of the block, one column per thread (zeros past w, in
-        // whole groups of 8), in whole warps: lanes 0..7 hold the reciprocals
-        if (warp * 32 < rem) {
+        // the 8 pivot rows right of the block, one column per thread (zeros past w), in
+        // whole warps: lanes 0..7 hold the reciprocals.  (The shuffle tells the compiler
+        // that a warp takes the branch as one: n = 3333 5875 -> 5795 us.)
+        if (__shfl_sync(0xffffffffu, warp, 0) * 32 < rem) {
             const int col = blk + CL_B + tid;
             const T dl = sh.d[blk + (lane & (CL_B - 1))], il = cl_zero(dl) ? T(1) : T(1) / dl;
             T x[CL_B], lij[CL_B][CL_B];
@@ -638,7 +639,7 @@ __global__ void __launch_bounds__(CL_ALL, 1) cluster_leaf_kernel(const CLeafPara
                 v *= __shfl_sync(0xffffffffu, il, j);
                 if (rank == 0 && tid < rem) P.a[(size_t)(c0 + blk + j) * P.ld + c0 + col] = v;
                 x[j] = cl_zero(__shfl_sync(0xffffffffu, dl, j)) ? T(0) : v;  // a zero pivot's column subtracts nothing
-                if (tid < ((rem + 7) & ~7)) cl_st1(ub + (j * C::UP + tid) * ES, x[j]);
+                if (W > 16 || tid < 8) cl_st1(ub + (j * C::UP + tid) * ES, x[j]);  // (16 columns: at most 8 of them)
             }
         }
         __syncthreads();
