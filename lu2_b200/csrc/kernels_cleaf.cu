@@ -753,29 +753,42 @@ static bool cl_prepare_1()
 }
 
 template <typename T, int W, bool TALL = false>
-static bool cl_prepare()
+static bool cl_prepare(bool query)
 {
-    return cl_prepare_1<T, W, TALL, false>() && cl_prepare_1<T, W, TALL, true>();
+    if (query) return cl_prepare_1<T, W, TALL, false>() && cl_prepare_1<T, W, TALL, true>();
+    return cl_attributes<T, W, TALL, false>() == cudaSuccess && cl_attributes<T, W, TALL, true>() == cudaSuccess;
 }
 
-// whether the current device takes the cluster leaf (looked up once per device)
-static bool cl_device_ok()
+// whether a device takes the cluster leaf: 0 not asked yet, else 1 or -1
+static std::atomic<signed char> cl_known[128];
+
+// The instances' sizes belong to the CUDA context and are gone after
+// cudaDeviceReset: set whenever a library context is made (for every launch they
+// cost the precision forms 0.5 us a leaf), the FP64 instances of up to 4096 rows
+// also by the allocation-free solve, which has none.
+bool cluster_leaf_setup(bool small)
 {
-    static std::atomic<signed char> known[128];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 128) return false;
-    signed char k = known[dev].load();
-    if (k == 0) {
-        k = cl_prepare<double, 64>() && cl_prepare<double, 32>() && cl_prepare<double, 16>() &&
-                    cl_prepare<float, 64>() && cl_prepare<float, 32>() && cl_prepare<float, 16>() &&
-                    cl_prepare<double, 32, true>() && cl_prepare<double, 16, true>() &&
-                    cl_prepare<float, 64, true>() && cl_prepare<float, 32, true>()
-                ? 1
-                : -1;
-        cudaGetLastError();
-        known[dev].store(k);
-    }
-    return k > 0;
+    const signed char known = cl_known[dev].load();
+    if (known < 0) return false;
+    const bool query = known == 0;
+    bool ok = cl_prepare<double, 64>(query) && cl_prepare<double, 32>(query) && cl_prepare<double, 16>(query);
+    if (!small || query)
+        ok = ok && cl_prepare<float, 64>(query) && cl_prepare<float, 32>(query) && cl_prepare<float, 16>(query) &&
+             cl_prepare<double, 32, true>(query) && cl_prepare<double, 16, true>(query) &&
+             cl_prepare<float, 64, true>(query) && cl_prepare<float, 32, true>(query);
+    if (query) cl_known[dev].store(ok ? 1 : -1);
+    cudaGetLastError();
+    return ok;
+}
+
+static bool cl_device_ok()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 128) return false;
+    const signed char known = cl_known[dev].load();
+    return known ? known > 0 : cluster_leaf_setup(false);
 }
 
 // columns the leaf takes for `rows` rows, in the tall instance or not; 0: not this leaf
@@ -811,10 +824,6 @@ static cudaError_t cl_launch_1(CLeafParams<T> P, cudaStream_t st)
     while (cl < 16 && cl * C::ROWS < rows) cl *= 2;
     P.rpc = (rows + cl - 1) / cl;
     if (P.rpc > C::ROWS) return cudaErrorInvalidConfiguration;
-    // set for every launch, as they belong to the CUDA context and not to the
-    // device: they are gone after cudaDeviceReset
-    const cudaError_t e = cl_attributes<T, W, TALL, REF>();
-    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)cl);
     cfg.blockDim = dim3(CL_ALL);

@@ -305,6 +305,7 @@ int leaf_max_ctas(int device)
     cudaFuncSetAttribute(leaf_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, leaf_kernel<double>, LEAF_THREADS, LEAF_SMEM_MAX);
     if (per_sm < 1) per_sm = 1;
+    cluster_leaf_setup(false);
     return sms * per_sm;
 }
 

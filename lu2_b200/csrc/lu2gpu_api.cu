@@ -1993,6 +1993,7 @@ static int noalloc_setup(int device, unsigned char **base, int *leaf_ctas)
                   cudaGetErrorString(e));
         return LU2GPU_ERR_CUDA;
     }
+    cluster_leaf_setup(true);  // belongs to it, too
     if (!g_noalloc_ctas[device]) {
         const int ctas = leaf_max_ctas(device);
         g_noalloc_ctas[device] = ctas < NOALLOC_LEAF_CTAS ? ctas : NOALLOC_LEAF_CTAS;

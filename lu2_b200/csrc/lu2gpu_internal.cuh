@@ -150,6 +150,9 @@ cudaError_t launch_leaf(double *a, long ld, int n, int c0, int w, int mode, int 
 cudaError_t launch_leaf(float *a, long ld, int n, int c0, int w, int mode, int goff, int *ipiv, float *dinv,
                         const LeafBuffers &buf, int *status, int max_ctas, cudaStream_t st);
 int leaf_max_ctas(int device);
+// sizes of the cluster leaf's instances in the current CUDA context (small: those of
+// the allocation-free solve); false where the device does not take it
+bool cluster_leaf_setup(bool small);
 // widest leaf for a panel of `rows` rows (elements of tsize bytes) with at most max_ctas CTAs
 int leaf_width(int rows, size_t tsize, int max_ctas);
 // the leaf on one thread-block cluster (kernels_cleaf.cu); *used = false, and
