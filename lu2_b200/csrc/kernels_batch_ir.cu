@@ -491,11 +491,6 @@ batch_ir_kernel(double *data, const BatchSys *sys, const long long *woff, uint8_
             for (int idx = tid; idx < n * r; idx += T) X[idx] = 0.0;
             __syncthreads();
             ir_residual(A, S.ld, n, r, X, R, true, s_red, s_rmax, s_xmax, s_bmax, &s_anorm);
-            // lu2's bar of 16 with room for the rounding of a residual: summed in any order
-            // it is off by at most (n + 1) u (|A||x| + |b|), (n + 1) / n in units of h, here
-            // and where the caller sums it (held to 16 itself, 1 of 20,000 systems came back
-            // at 16.01)
-            const double bar = 16.0 - 2.0 * (n + 1) / n;
             for (it = 1; it <= max_iter; it++) {
                 for (int i = tid; i < n; i += T) {
                     const int from = perm[i];
@@ -507,8 +502,13 @@ batch_ir_kernel(double *data, const BatchSys *sys, const long long *woff, uint8_
                 ir_residual(A, S.ld, n, r, X, R, false, s_red, s_rmax, s_xmax, s_bmax, &s_anorm);
                 if (tid == 0) {
                     bool ok = true;
+                    // lu2's bar of 16 with room for the rounding of a residual: summed with k
+                    // roundings it is off by at most k u (|A||x| + |b|), k / n in units of h; k
+                    // is at most n / 64 + 9 here and n + 1 wherever the caller sums it (held
+                    // to 16 itself, 1 of 20,000 systems came back at 16.01)
+                    const double bar = 16 * n - (n + 1 + min(n + 1, n / 64 + 9));  // of n h
                     for (int q = 0; q < r; q++) {
-                        const double h = s_rmax[q] / (1.1102230246251565e-16 * (s_anorm * s_xmax[q] + s_bmax[q]) * n);
+                        const double h = s_rmax[q] / (1.1102230246251565e-16 * (s_anorm * s_xmax[q] + s_bmax[q]));
                         if (!(h < bar)) ok = false;
                     }
                     s_done = ok;
