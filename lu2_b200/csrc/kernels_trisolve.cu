@@ -522,6 +522,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) tri_solve_kernel(const TriParam
                                   (*(volatile int *)&P.status[1] != 0 || globaltimer_ns() - t0 > WAIT_LIMIT_NS);
                 if ((round & 63u) == 0 && __syncthreads_or(late)) {
                     if (tid == 0 && *(volatile int *)&P.status[1] == 0) record_error(P.status, ERR_BARRIER_TIMEOUT, 6);
+                    asm volatile("cp.async.wait_all;" ::: "memory");  // the next diagonal block, on its way to Td
                     return;
                 }
             }
