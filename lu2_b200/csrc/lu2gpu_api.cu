@@ -2159,7 +2159,8 @@ struct View32 {
 // onto the GPU before the update's CTAs: a leaf's cluster needs 16 free SMs side
 // by side, finds none once the persistent update lies on all parts of the GPU
 // (the panel then waited for the whole update), and leaves them free for the
-// panel's next leaves.
+// panel's next leaves.  Nothing guarantees it: a side stream whose launch comes
+// late costs that panel the rest of the update, never a result.
 template <typename Hook>
 static int right_part32_split(lu2gpu_ctx *c, const View32 &v, int k0, int k1, int cs, int ce, int w1, int max_ctas,
                               SwapJobs left, Hook after_first);
