@@ -653,7 +653,10 @@ static int ts_sms()
 // Right-hand sides (FP64) up to which the two persistent solves beat the panel
 // loop.  A pass of 8 walks the chain of blocks again; the loop's panels cost about
 // the same for any of these numbers.  us, persistent / panel loop:
-//   one block (n = 100, panels of 128):  8: 73 / 68, 16: 104 / 82; of 16:  16: 152 / 163, 24: 207 / 178
+//   one panel, n = 16:  1: 56 / 50, 8: 59 / 51;  64:  1: 57 / 55, 8: 64 / 58 (the row map, two launches, is more
+//       than one exchange);  96:  1: 60.6 / 61.0, 4: 61.4 / 62.1, 8: 70 / 66;  128:  1: 62 / 66, 4: 65 / 66, 8: 76 / 73
+//   one block of several panels, n = 17, panels of 16:  1: 58 / 63, 8: 62 / 66;  96, of 64:  1: 63 / 75, 8: 73 / 79;
+//       100, of 16:  16: 152 / 163, 24: 207 / 178
 //   panels of 512, n = 4096:  32: 3293 / 3779 (the loop's block solves are slow there)
 //   256:  17: 2044 / 1975 (n = 40000: 20.6 / 21.8 ms), 24: 2463 / 2167
 //   128:  17: 2034 / 2115, 24: 2452 / 2279;  64:  17: 2361 / 2427, 24: 2814 / 2636
@@ -664,6 +667,7 @@ static int ts_sms()
 // (a block is never larger than a panel, and one of 16 rows costs a tile of 128)
 int tri_solve_few_rhs(int n, int nb)
 {
+    if (n <= nb && n <= TS_B) return n <= 64 ? 0 : 4;
     if (n <= TS_B) return nb >= 48 ? BS_MAXR : 16;
     if (nb > 256) return 32;
     if (nb >= 48) return nb >= 64 ? 18 : 16;
